@@ -123,7 +123,8 @@ typedef struct flk_batch flk_batch;
 
 /* An empty batch on `device` (< 0: the current device); no counterpart. */
 int flk_batch_create(int32_t device, flk_batch** out);
-/* Adds a flock (as flk_open_host); *id receives its handle within the batch. */
+/* Adds a flock (as flk_open_host: `words` has been read when the call returns);
+ * *id receives its handle within the batch. */
 int flk_batch_add(flk_batch* b, uint32_t n, float time, const float* words, int32_t* id);
 /* Drops a flock and frees its storage for later flocks; no counterpart. */
 int flk_batch_remove(flk_batch* b, int32_t id);

@@ -108,7 +108,7 @@ extern "C" int flk_open_host(int32_t device, uint32_t n, float time, const float
     return guarded([&] {
         auto f = std::make_unique<flk_flock>();
         f->eng = std::make_unique<Engine>(device);
-        f->id = f->eng->add_flock(n, time, words, true);
+        f->id = f->eng->add_flock(n, time, words);
         f->n = n;
         *out = f.release();
         return FLK_OK;

@@ -506,7 +506,7 @@ void Engine::ensure_arena(uint32_t need) {
     free_graphs();
 }
 
-int Engine::add_flock(uint32_t n, float time, const float* words, bool wait) {
+int Engine::add_flock(uint32_t n, float time, const float* words) {
     FLK_CUDA(cudaSetDevice(device_));
     // first-fit into a hole, else append
     uint32_t sbase = used_;
@@ -529,7 +529,7 @@ int Engine::add_flock(uint32_t n, float time, const float* words, bool wait) {
                        free_ranges_.end());
     if (n) {
         const size_t bytes = (size_t)n * WORDS * 4;
-        const float* src = wait ? static_cast<const float*>(mapped(words, bytes)) : nullptr;
+        const float* src = static_cast<const float*>(mapped(words, bytes));
         if (!src) {  // by way of a staging copy
             ensure_staging(bytes);
             FLK_CUDA(cudaMemcpyAsync(staging_, words, bytes, cudaMemcpyHostToDevice, stream_));
@@ -537,7 +537,9 @@ int Engine::add_flock(uint32_t n, float time, const float* words, bool wait) {
         }
         k_unpack<<<pack_blocks(n), PACK_WARPS * 32, 0, stream_>>>(src, n, sbase, ar_);  // buffer 0
         FLK_CUDA(cudaGetLastError());
-        if (wait) FLK_CUDA(cudaStreamSynchronize(stream_));
+        // page-locked words are read after the launches return: the caller may
+        // change them, or give their memory back, as soon as this call does
+        FLK_CUDA(cudaStreamSynchronize(stream_));
     }
     Slot s;
     s.n = n;

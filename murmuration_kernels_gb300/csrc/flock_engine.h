@@ -112,10 +112,9 @@ public:
     Engine(const Engine&) = delete;
     Engine& operator=(const Engine&) = delete;
 
-    // Flocks. `words` is a host array of n*15 .flk words (any host memory).
-    // wait: return when they have been read (straight from page-locked memory),
-    // otherwise their copy may still be in flight where they are page-locked.
-    int add_flock(uint32_t n, float time, const float* words, bool wait = false);  // returns id >= 0
+    // Flocks. `words` is a host array of n*15 .flk words (any host memory), which
+    // has been read when the call returns.
+    int add_flock(uint32_t n, float time, const float* words);  // returns id >= 0
     // Same, but the host-to-device copy runs on the copy stream and overlaps
     // the compute stream's work; `words` must stay valid until the next sync.
     int add_flock_async(uint32_t n, float time, const float* words);
