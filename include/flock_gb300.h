@@ -278,7 +278,8 @@ int flk_pin(void* ptr, uint64_t bytes);
 int flk_unpin(void* ptr);
 /* A page-locked buffer of at least `bytes` for results or states, from a
  * process-wide bounded cache, and its return to it (locking pages afresh costs
- * about a millisecond per 10 MB); safe from any thread. No counterpart. */
+ * about a millisecond per 25 MB); safe from any thread. Private memory: a
+ * forked child has its own copy. No counterpart. */
 int flk_host_alloc(uint64_t bytes, void** ptr);
 void flk_host_free(void* ptr);
 
