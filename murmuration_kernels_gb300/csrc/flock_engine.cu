@@ -298,8 +298,11 @@ void Engine::dfree(T*& p) {
 }
 
 // The device address of page-locked host memory [p, p + bytes), or null where
-// its first or last byte is not page-locked (or not one mapping).
+// its first or last byte is not page-locked (or not one mapping), and where the
+// kernels' 4-byte words would not be aligned (a float32 view at an odd byte
+// offset: the copy engine takes any address, a load or store does not).
 static void* mapped(const void* p, size_t bytes) {
+    if (reinterpret_cast<uintptr_t>(p) % sizeof(float)) return nullptr;
     auto at = [](const void* q) -> char* {
         cudaPointerAttributes a{};
         if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
