@@ -276,6 +276,10 @@ int flk_kernels_per_step(void);
  * reference copies from pageable vectors, cuda/flock.cu:414-437). */
 int flk_pin(void* ptr, uint64_t bytes);
 int flk_unpin(void* ptr);
+/* 1 where states in host memory [ptr, ptr + bytes) cross the link straight from
+ * and to it: 4-byte aligned and within one page-locked range. Otherwise 0: they
+ * go through a staging buffer. No counterpart. */
+int flk_copies_straight(const void* ptr, uint64_t bytes);
 /* A page-locked buffer of at least `bytes` for results or states, from a
  * process-wide bounded cache, and its return to it (locking pages afresh costs
  * about a millisecond per 25 MB); safe from any thread. Private memory: a

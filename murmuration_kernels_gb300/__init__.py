@@ -118,6 +118,7 @@ _SIGS = {
     "flk_kernels_per_step": (C.c_int, []),
     "flk_pin": (C.c_int, [C.c_void_p, C.c_uint64]),
     "flk_unpin": (C.c_int, [C.c_void_p]),
+    "flk_copies_straight": (C.c_int, [C.c_void_p, C.c_uint64]),
     "flk_host_alloc": (C.c_int, [C.c_uint64, C.POINTER(C.c_void_p)]),
     "flk_host_free": (None, [C.c_void_p]),
 }

@@ -1003,6 +1003,14 @@ extern "C" int flk_unpin(void* ptr) {
     return FLK_OK;
 }
 
+extern "C" int flk_copies_straight(const void* ptr, uint64_t bytes) {
+    try {
+        return flk::mapped(ptr, (size_t)bytes) != nullptr;
+    } catch (...) {
+        return 0;
+    }
+}
+
 extern "C" int flk_host_alloc(uint64_t bytes, void** ptr) {
     if (!ptr || !bytes) return fail(FLK_ERR_ARG, "flk_host_alloc: null pointer or zero size");
     return guarded([&] {

@@ -37,6 +37,7 @@
 // keys, the sorted order and all four neighbour sets equal the CPU oracle's
 // bit for bit. Sums run in lane order instead of bird order, so forces agree
 // to rounding (about 1e-7 relative), not bit for bit.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <sys/mman.h>
 #include <unistd.h>
@@ -297,22 +298,36 @@ void Engine::dfree(T*& p) {
     p = nullptr;
 }
 
-// The device address of page-locked host memory [p, p + bytes), or null where
-// its first or last byte is not page-locked (or not one mapping), and where the
-// kernels' 4-byte words would not be aligned (a float32 view at an odd byte
+// The device address of host memory [p, p + bytes) that lies in one page-locked
+// range, or null: where it is not page-locked, only part of it is (two
+// registrations may lie within it and pages between them that a kernel must not
+// touch; device addresses equal host addresses, so the ends alone do not tell),
+// or the kernels' 4-byte words would not be aligned (a float32 view at an odd byte
 // offset: the copy engine takes any address, a load or store does not).
-static void* mapped(const void* p, size_t bytes) {
-    if (reinterpret_cast<uintptr_t>(p) % sizeof(float)) return nullptr;
-    auto at = [](const void* q) -> char* {
-        cudaPointerAttributes a{};
-        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+void* mapped(const void* p, size_t bytes) {
+    using Query = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found) !=
+                cudaSuccess || found != cudaDriverEntryPointSuccess) {
             (void)cudaGetLastError();
-            return nullptr;
+            f = nullptr;
         }
-        return a.type == cudaMemoryTypeHost ? static_cast<char*>(a.devicePointer) : nullptr;
-    };
-    char* first = at(p);
-    return first && at((const char*)p + bytes - 1) == first + (bytes - 1) ? first : nullptr;
+        return reinterpret_cast<Query>(f);
+    }();
+    if (!query || reinterpret_cast<uintptr_t>(p) % sizeof(float)) return nullptr;
+    unsigned int type = 0, managed = 0;
+    unsigned long long at = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* to[] = {&type, &managed, &at, &start, &size};
+    if (query(5, what, to, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return nullptr;
+    if (type != CU_MEMORYTYPE_HOST || managed || !at || at < start) return nullptr;
+    const size_t before = (size_t)(at - start);
+    return before < size && bytes <= size - before ? reinterpret_cast<void*>((uintptr_t)at) : nullptr;
 }
 
 Engine::Engine(int device) {

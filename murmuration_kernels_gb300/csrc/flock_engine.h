@@ -313,6 +313,8 @@ uint32_t production_buckets(uint32_t n);
 // Page-locked host blocks from a bounded cache (null where the host gives none).
 void* host_alloc(size_t bytes);
 void host_free(void* p);
+// Where kernels may access host memory [p, p + bytes) directly, or null.
+void* mapped(const void* p, size_t bytes);
 
 // What a device error word (DeviceError) means, as FLK_ERR_DEVICE reports it.
 const char* device_error_text(uint32_t word);
