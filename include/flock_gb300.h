@@ -248,6 +248,11 @@ const char* flk_device_error_text(uint32_t word);
  * leaves the flock's state unusable (close it); the device and the process
  * stay usable. No fault, trap or unbounded wait is involved. */
 int flk_debug_scan_timeout(flk_flock* f, uint32_t skip_tile, uint32_t spin_limit);
+/* Test hook for failing CUDA graph calls, on the host alone; no counterpart. The
+ * flock's next `captures` graph captures fail (its steps then go launch by
+ * launch), and so does the `launch`-th graph launch from now (0: none), which
+ * ends that flk_step with FLK_ERR_CUDA after whole steps; the flock stays usable. */
+int flk_debug_fail_graphs(flk_flock* f, uint32_t captures, uint32_t launch);
 
 /* ---- helpers -------------------------------------------------------------- */
 /* The calling thread's last error message: what the CK macro prints before

@@ -77,6 +77,7 @@ _SIGS = {
     "flk_decide_occupancy": (C.c_int, [_P, C.c_uint64, _PI, _PI, _PI, _PU64]),
     "flk_device_error_text": (C.c_char_p, [C.c_uint32]),
     "flk_debug_scan_timeout": (C.c_int, [_P, C.c_uint32, C.c_uint32]),
+    "flk_debug_fail_graphs": (C.c_int, [_P, C.c_uint32, C.c_uint32]),
     "flk_step_debug": (C.c_int, [_P, _PU, _PU, _PU, _PU]),
     "flk_counters": (C.c_int, [_P, _PU64, _PU64, _PU64]),
     "flk_step_f64": (C.c_int, [_P, _PD, _PD]),
@@ -351,6 +352,10 @@ class Flock:
     def debug_scan_timeout(self, skip_tile: int = 0, spin_limit: int = 1000) -> None:
         """Test hook: the next step_debug's scan gives up waiting (FLK_ERR_DEVICE)."""
         _check(lib().flk_debug_scan_timeout(self._h, skip_tile, spin_limit))
+
+    def debug_fail_graphs(self, captures: int = 0, launch: int = 0) -> None:
+        """Test hook: the next graph captures, and the launch-th graph launch, fail."""
+        _check(lib().flk_debug_fail_graphs(self._h, captures, launch))
 
     def time_steps(self, steps: int, flush_bytes: int = 256 << 20) -> np.ndarray:
         """Device ms of each of `steps` single-step launches, L2 flushed before each.

@@ -200,6 +200,12 @@ extern "C" int flk_debug_scan_timeout(flk_flock* f, uint32_t skip_tile, uint32_t
     });
 }
 
+extern "C" int flk_debug_fail_graphs(flk_flock* f, uint32_t captures, uint32_t launch) {
+    if (!f) return fail(FLK_ERR_ARG, "flk_debug_fail_graphs: null handle");
+    f->eng->fail_graphs(captures, launch);
+    return FLK_OK;
+}
+
 extern "C" int flk_size(const flk_flock* f, uint32_t* n, uint32_t* buckets) {
     if (!f) return fail(FLK_ERR_ARG, "flk_size: null handle");
     if (n) *n = f->n;

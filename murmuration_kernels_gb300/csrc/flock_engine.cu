@@ -1034,6 +1034,7 @@ void Engine::enqueue_step(bool sets, cudaEvent_t* ev, bool f64, bool hash, bool 
     const uint32_t ntiles = Btot_ / SCAN_TILE;
     const float cell = shape_.cell, inv_cell = 1.0f / shape_.cell;  // production cells
     if (ev) FLK_CUDA(cudaEventRecord(ev[0], stream_));
+    if (sets) clear_counted();
     if (sets)  // a grid-reporting step: the reference's cell hash
         k_hash_count<false><<<sgrid(fit_.hash[0]), 256, 0, stream_>>>(table_d_, nfl, V_, ar_, key_, arrival_, counts_,
                                                                       INV_CELL);
@@ -1079,15 +1080,25 @@ void Engine::enqueue_step(bool sets, cudaEvent_t* ev, bool f64, bool hash, bool 
     else
         k_integrate<false><<<sgrid(fit_.integrate[0]), 256, 0, stream_>>>(table_d_, nfl, V_, ar_, counts_, key_,
                                                                           arrival_, ctl_, inv_cell, move);
+    counted_ = fuse_next && !sets;
     if (f64) k_compare_f64<<<sgrid(fit_.compare_f64), 256, 0, stream_>>>(table_d_, nfl, V_, ar_, active_, out64_, err64_);
     if (ev) FLK_CUDA(cudaEventRecord(ev[5], stream_));
 }
 
+// A run that failed between two steps has left the next step's grid counted.
+void Engine::clear_counted() {
+    if (!counted_) return;
+    FLK_CUDA(cudaMemsetAsync(counts_, 0, (size_t)scratch_B_ * 4, stream_));
+    counted_ = false;
+}
+
 void Engine::enqueue_hash() {
     device_ahead_ = true;
+    clear_counted();
     const int grid = pgrid(num_sms_, std::min(shape_.stream_blocks_per_sm, fit_.hash[1]), V_, 256);
     k_hash_count<true><<<grid, 256, 0, stream_>>>(table_d_, (int)table_h_.size(), V_, ar_, key_, arrival_, counts_,
                                                   1.0f / shape_.cell);
+    counted_ = true;
 }
 
 void Engine::enqueue_steps(uint32_t n) {
@@ -1133,30 +1144,49 @@ void Engine::enqueue_small(uint32_t steps, uint32_t ctas) {
 // instantiating a new one (launches already in flight keep their old
 // parameters). A different length, or an update the runtime refuses,
 // instantiates afresh.
-void Engine::ensure_graph(StepGraph& sg, uint32_t steps) {
-    if (sg.exec && sg.steps == steps && !sg.stale) return;
-    cudaGraph_t g;
-    FLK_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+// False where the runtime gives no graph: the steps then go launch by launch. Called
+// when no grid is counted, or before: a capture that fails changes nothing.
+bool Engine::ensure_graph(StepGraph& sg, uint32_t steps) {
+    if (sg.exec && sg.steps == steps && !sg.stale) return true;
+    const auto failed = [] {
+        (void)cudaGetLastError();  // leaves no sticky error
+        return false;
+    };
+    if (fail_captures_) return --fail_captures_, false;
+    cudaGraph_t g = nullptr;
+    if (cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return failed();
+    const bool counted = counted_;
+    counted_ = false;
     if (&sg == &step_graph_) enqueue_step(false, nullptr, false, false, true, false);
     else enqueue_steps(steps);
-    FLK_CUDA(cudaStreamEndCapture(stream_, &g));
+    counted_ = counted;
+    if (cudaStreamEndCapture(stream_, &g) != cudaSuccess) return failed();
     if (sg.exec && sg.steps == steps) {
         cudaGraphExecUpdateResultInfo info;
         if (cudaGraphExecUpdate(sg.exec, g, &info) == cudaSuccess) {
             cudaGraphDestroy(g);
             sg.stale = false;
             ++graph_updates_;
-            return;
+            return true;
         }
         (void)cudaGetLastError();  // the refused update leaves no sticky error
     }
     if (sg.exec) cudaGraphExecDestroy(sg.exec);
     sg = StepGraph{};
-    cudaError_t e = cudaGraphInstantiate(&sg.exec, g, 0);
+    const cudaError_t e = cudaGraphInstantiate(&sg.exec, g, 0);
     cudaGraphDestroy(g);
-    FLK_CUDA(e);
+    if (e != cudaSuccess) {
+        sg = StepGraph{};
+        return failed();
+    }
     sg.steps = steps;
     ++graph_instantiations_;
+    return true;
+}
+
+void Engine::launch_graph(const StepGraph& sg) {
+    if (fail_launch_ && --fail_launch_ == 0) throw Error{-3, "graph launch failed (test hook)"};
+    FLK_CUDA(cudaGraphLaunch(sg.exec, stream_));
 }
 
 // A kernel launch takes the host about 7 us, a graph launch no more, and a
@@ -1180,12 +1210,13 @@ void Engine::enqueue_run(uint32_t steps) {
             if (!ready) {
                 enqueue_singly(chunk);
                 done = chunk;
-                ensure_graph(chunk_graph_, chunk);
             }
-            for (; done + chunk <= steps; done += chunk) FLK_CUDA(cudaGraphLaunch(chunk_graph_.exec, stream_));
-            since_move_ = (chunk - 1) % MOVE_EVERY + 1;  // a chunk's first step moves the state
-            for (int id : table_ids_)
-                if (id >= 0) slots_[id].fresh = false;
+            if (ensure_graph(chunk_graph_, chunk)) {
+                for (; done + chunk <= steps; done += chunk) launch_graph(chunk_graph_);
+                since_move_ = (chunk - 1) % MOVE_EVERY + 1;  // a chunk's first step moves the state
+                for (int id : table_ids_)
+                    if (id >= 0) slots_[id].fresh = false;
+            }
         }
         ++same_runs_;
     }
@@ -1198,7 +1229,8 @@ void Engine::enqueue_run(uint32_t steps) {
 void Engine::enqueue_singly(uint32_t n) {
     for (int id : table_ids_)
         if (id >= 0 && slots_[id].fresh) since_move_ = MOVE_EVERY;
-    const bool graphed = n >= 4 || (n >= 2 && step_graph_.exec && !step_graph_.stale);
+    // the graph before any grid is counted: a failing capture must not leave one
+    const bool graphed = (n >= 4 || (n >= 2 && step_graph_.exec && !step_graph_.stale)) && ensure_graph(step_graph_, 1);
     for (uint32_t i = 0; i < n; ++i) {
         const bool last = i + 1 == n, move = since_move_ >= MOVE_EVERY;
         if (move) {
@@ -1212,8 +1244,7 @@ void Engine::enqueue_singly(uint32_t n) {
             continue;
         }
         if (i == 0) enqueue_hash();
-        ensure_graph(step_graph_, 1);
-        FLK_CUDA(cudaGraphLaunch(step_graph_.exec, stream_));
+        launch_graph(step_graph_);
     }
 }
 

@@ -164,6 +164,12 @@ public:
     // gives up after `spin_limit` polls (0: the usual limit). The step then
     // ends with the device error word set to DEV_SCAN_TIMEOUT.
     void arm_scan_timeout(uint32_t skip_tile, uint32_t spin_limit);
+    // Test hook for the host's failure paths: the next `captures` graph captures
+    // fail, and so does the `launch`-th graph launch from now (0: none).
+    void fail_graphs(uint32_t captures, uint32_t launch) {
+        fail_captures_ = captures;
+        fail_launch_ = launch;
+    }
 
     cudaStream_t stream() const { return stream_; }
     int device() const { return device_; }
@@ -229,7 +235,9 @@ private:
     };
     void free_graphs();
     void destroy_graphs();
-    void ensure_graph(StepGraph& g, uint32_t steps);
+    bool ensure_graph(StepGraph& g, uint32_t steps);
+    void launch_graph(const StepGraph& g);
+    void clear_counted();
     void enqueue_run(uint32_t steps);
     void enqueue_singly(uint32_t n);
     void ensure_block(uint32_t flocks);
@@ -303,6 +311,8 @@ private:
     uint32_t since_move_ = 0;  // steps since the state was last moved into cell order
     uint32_t same_runs_ = 0;  // runs of at least a chunk since the table's shape changed
     uint64_t graph_instantiations_ = 0, graph_updates_ = 0;
+    bool counted_ = false;  // the histogram holds a grid that the next step enqueued will use
+    uint32_t fail_captures_ = 0, fail_launch_ = 0;  // fail_graphs
 };
 
 // Canonical bucket count for a flock of n birds (reference cuda/flock.cu:368-372).
