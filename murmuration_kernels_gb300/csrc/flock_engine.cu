@@ -1125,6 +1125,7 @@ uint32_t Engine::small_ctas() const {
     return 0;
 }
 
+// A launch runs at most SMALL_STEPS steps, 0.1 s or so.
 void Engine::enqueue_small(uint32_t steps, uint32_t ctas) {
     device_ahead_ = true;
     uint32_t nmax = 1;
@@ -1132,8 +1133,12 @@ void Engine::enqueue_small(uint32_t steps, uint32_t ctas) {
     cudaLaunchAttribute at{};
     cudaLaunchConfig_t c = small_config((uint32_t)table_h_.size(), ctas, nmax, &at);
     c.stream = stream_;
-    FLK_CUDA(cudaLaunchKernelEx(&c, k_small, table_d_, steps, nmax, ctl_, ar_, (const float*)radius_table_, shape_.cell,
-                                1.0f / shape_.cell));
+    for (uint32_t done = 0; done < steps;) {
+        const uint32_t part = std::min(steps - done, SMALL_STEPS);
+        FLK_CUDA(cudaLaunchKernelEx(&c, k_small, table_d_, part, nmax, ctl_, ar_, (const float*)radius_table_,
+                                    shape_.cell, 1.0f / shape_.cell));
+        done += part;
+    }
 }
 
 // Captures `steps` production steps (1: the step alone, its grid counted before

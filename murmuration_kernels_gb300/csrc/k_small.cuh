@@ -40,6 +40,11 @@ constexpr int SMALL_SIZES = 5;  // cluster sizes: SMALL_CTAS >> 0 .. 4
 // step, this kernel against the separate ones: 500 birds 5.9 / 17.7, 2,000
 // 10.2 / 20.2, 3,000 12.5 / 22, 4,096 16 / 22).
 constexpr uint32_t SMALL_CLUSTER = 4096;
+// Steps of one launch, at most, which keeps a warp's 32-bit counters from running
+// over (each of its birds deciding every step with every bird a candidate) and
+// bounds a kernel's time.
+constexpr uint32_t SMALL_STEPS = 8192;
+static_assert((uint64_t)SMALL_STEPS * 32u * SMALL_CLUSTER < 1ull << 32, "32 birds a warp at most");
 constexpr uint32_t SMALL_BUCKETS = 8192;                          // every such flock's bucket count
 constexpr uint32_t SMALL_PER = SMALL_CLUSTER / SMALL_THREADS;  // birds a thread sorts, at most
 static_assert(SMALL_CLUSTER <= SMALL_FLOCK, "the decisions are a warp per bird");
