@@ -309,9 +309,14 @@ void flk_host_free(void* ptr);
  * FLK_NOALLOC_MAX_BIRDS birds; larger n returns FLK_ERR_CAPACITY. Each call
  * looks up that array's device address on the current device. n = 0 still
  * writes all buckets_for(0)+1 = 65,537 offsets (zeros). Calls share the array:
- * concurrent calls on one device race. */
+ * concurrent calls on one device race. The first call page-locks one page of the
+ * library's own host memory, for the kernel's error word. */
 #define FLK_NOALLOC_MAX_BIRDS 131072u
 int flk_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets, uint32_t* sorted, void* stream);
+/* Test hook: the same call by separate launches, as where the device cannot hold
+ * the one kernel's blocks at once (`separate`). */
+int flk_debug_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets, uint32_t* sorted,
+                           void* stream, int32_t separate);
 
 #ifdef __cplusplus
 }

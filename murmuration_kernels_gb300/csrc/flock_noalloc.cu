@@ -55,9 +55,11 @@ constexpr uint32_t FULL = 0xFFFFFFFFu;
 // Byte layout of the scratch array (each region 256-byte aligned).
 constexpr size_t OFF_COUNTS = 0;                                  // MAX_BUCKETS u32
 constexpr size_t OFF_TMP = OFF_COUNTS + MAX_BUCKETS * 4ull;       // MAX_BIRDS u32
-constexpr size_t OFF_CTL = OFF_TMP + MAX_BIRDS * 4ull;            // 128 u32
-constexpr size_t SCRATCH_BYTES = OFF_CTL + 512;
-enum { CTL_ERROR = 0, CTL_ARRIVED = 8, CTL_TURN = 16, CTL_SUM = 64 };  // an error; the barrier; birds per tile
+constexpr size_t OFF_CTL = OFF_TMP + MAX_BIRDS * 4ull;            // CTL_WORDS u32
+// an error; birds per tile; the barrier's counters (arrived, turns)
+enum { CTL_ERROR = 0, CTL_SUM = 64, CTL_BARRIER = 128, CTL_WORDS = CTL_BARRIER + 16 };
+enum { ARRIVED = 0, TURN = 8 };
+constexpr size_t SCRATCH_BYTES = OFF_CTL + CTL_WORDS * 4ull;
 constexpr int THREADS = 1024;        // per CTA
 constexpr uint32_t TILE = 4096;      // buckets per CTA in the scan
 constexpr uint32_t SPIN_LIMIT = 1u << 20;  // polls of a barrier before it gives up
@@ -83,7 +85,7 @@ Scratch carve(unsigned char* base) {
 
 __device__ __forceinline__ int cell1(float x) { return (int)floorf(__fmul_rn(x, flk::INV_CELL)); }
 
-// Loads of what another CTA of the cluster wrote in an earlier phase.
+// Loads of what another CTA wrote in an earlier phase.
 __device__ __forceinline__ uint32_t ld(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -100,16 +102,16 @@ __device__ __forceinline__ uint4 ld(const uint4* p) {
 // Orders every earlier access of the grid's threads before every later one (a
 // cooperative launch: all CTAs are resident). The wait is bounded: false, in
 // every thread of a CTA, where it gave up.
-__device__ __forceinline__ bool grid_barrier(uint32_t* ctl, uint32_t* status) {
+__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t* status) {
     __shared__ uint32_t s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile uint32_t* turn = ctl + CTL_TURN;
+        volatile uint32_t* turn = bar + TURN;
         const uint32_t now = *turn;
         uint32_t polls = 0;
         __threadfence();
-        if (atomicAdd(&ctl[CTL_ARRIVED], 1u) == gridDim.x - 1u) {
-            ctl[CTL_ARRIVED] = 0;
+        if (atomicAdd(&bar[ARRIVED], 1u) == gridDim.x - 1u) {
+            bar[ARRIVED] = 0;
             __threadfence();
             *turn = now + 1u;
         } else {
@@ -161,35 +163,48 @@ __device__ __forceinline__ void sort_bucket(const uint32_t* tmp, uint32_t s0, ui
     }
 }
 
+constexpr int PHASES = 5;  // clear, count, scan, scatter, order
+
 // buckets: a power of two of at least 2^16, and at least 2n; buckets / 2 threads.
 // *status: zero at the start, an error word where there was one.
+// FUSED: every phase (a cooperative launch); otherwise phase `arg` alone, the
+// arrival ranks waiting in `sorted` for the scatter.
+template <bool FUSED>
 __global__ void __launch_bounds__(THREADS, 1) k_na_grid(const float4* __restrict__ pos, uint32_t n, uint32_t buckets,
-                                                        uint32_t* __restrict__ keys, uint32_t* offsets,
-                                                        uint32_t* __restrict__ sorted, Scratch s, uint32_t* status) {
+                                                        uint32_t* keys, uint32_t* offsets, uint32_t* sorted, Scratch s,
+                                                        uint32_t* status, uint32_t arg) {
     __shared__ uint32_t s_warp[THREADS / 32], s_tile[MAX_BUCKETS / TILE];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, v = blockIdx.x * THREADS + tid;
     const bool mine = v < n;  // this thread's bird
-    reinterpret_cast<uint2*>(s.counts)[v] = make_uint2(0u, 0u);
-    if (v < MAX_BUCKETS / TILE) s.ctl[CTL_SUM + v] = 0;
+    uint32_t* bar = s.ctl + CTL_BARRIER;
+    const auto runs = [&](uint32_t phase) { return FUSED || arg == phase; };
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (mine) p = pos[v];
-    if (tid < MAX_BUCKETS / TILE) s_tile[tid] = 0;
-    if (!grid_barrier(s.ctl, status)) return;
-    // hash and count, each tile of buckets as a whole as well
     uint32_t b = 0, arrival = 0;
-    if (mine) {
-        b = (((uint32_t)cell1(p.x) * 73856093u) ^ ((uint32_t)cell1(p.y) * 19349663u) ^
-             ((uint32_t)cell1(p.z) * 83492791u)) & (buckets - 1u);
-        arrival = atomicAdd(&s.counts[b], 1u);
-        keys[v] = b;
-        atomicAdd(&s_tile[b / TILE], 1u);
+    if (mine && (FUSED || arg == 1)) p = pos[v];
+    if (tid < MAX_BUCKETS / TILE) s_tile[tid] = 0;
+    if (runs(0)) {
+        reinterpret_cast<uint2*>(s.counts)[v] = make_uint2(0u, 0u);
+        if (v < MAX_BUCKETS / TILE) s.ctl[CTL_SUM + v] = 0;
     }
-    __syncthreads();
-    if (tid < MAX_BUCKETS / TILE && s_tile[tid]) atomicAdd(&s.ctl[CTL_SUM + tid], s_tile[tid]);
-    if (!grid_barrier(s.ctl, status)) return;
+    if (FUSED && !grid_barrier(bar, status)) return;
+    // hash and count, each tile of buckets as a whole as well
+    if (runs(1)) {
+        if (!FUSED) __syncthreads();  // s_tile is clear
+        if (mine) {
+            b = (((uint32_t)cell1(p.x) * 73856093u) ^ ((uint32_t)cell1(p.y) * 19349663u) ^
+                 ((uint32_t)cell1(p.z) * 83492791u)) & (buckets - 1u);
+            arrival = atomicAdd(&s.counts[b], 1u);
+            keys[v] = b;
+            atomicAdd(&s_tile[b / TILE], 1u);
+            if (!FUSED) sorted[v] = arrival;
+        }
+        __syncthreads();
+        if (tid < MAX_BUCKETS / TILE && s_tile[tid]) atomicAdd(&s.ctl[CTL_SUM + tid], s_tile[tid]);
+    }
+    if (FUSED && !grid_barrier(bar, status)) return;
     // exclusive scan, a tile per CTA (half of the CTAs)
     const uint32_t tiles = buckets / TILE;  // 16 to 64
-    if (blockIdx.x < tiles) {
+    if (runs(2) && blockIdx.x < tiles) {
         const uint4 c = ld(reinterpret_cast<const uint4*>(s.counts + blockIdx.x * TILE) + tid);
         uint32_t before = 0;  // birds of the tiles before
         for (uint32_t t = lane; t < blockIdx.x; t += 32) before += ld(&s.ctl[CTL_SUM + t]);
@@ -206,16 +221,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_na_grid(const float4* __restrict
         reinterpret_cast<uint4*>(offsets + blockIdx.x * TILE)[tid] = o;
         if (blockIdx.x == tiles - 1 && tid == THREADS - 1) offsets[buckets] = run;
     }
-    if (!grid_barrier(s.ctl, status)) return;
+    if (FUSED && !grid_barrier(bar, status)) return;
     // scatter by arrival rank
-    if (mine) {
+    if (runs(3) && mine) {
+        if (!FUSED) {
+            b = keys[v];
+            arrival = sorted[v];
+        }
         const uint32_t to = ld(&offsets[b]) + arrival;
         if (to < n) s.tmp[to] = v;
         else *(volatile uint32_t*)status = 2u;
     }
-    if (!grid_barrier(s.ctl, status)) return;
+    if (FUSED && !grid_barrier(bar, status)) return;
     // each occupied bucket in bird order, a warp each; a warp looks through 32
     // buckets at a time, the CTAs' warps in turn
+    if (!runs(4)) return;
     for (uint32_t b0 = (warp * gridDim.x + blockIdx.x) * 32u; b0 < buckets; b0 += gridDim.x * THREADS) {
         const uint32_t s0 = ld(&offsets[b0 + lane]), L = ld(&s.counts[b0 + lane]);
         uint32_t some = __ballot_sync(FULL, L != 0);
@@ -253,10 +273,9 @@ int na_fail(int code, const std::string& m) {
     return code;
 }
 
-}  // namespace
-
-extern "C" int flk_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets, uint32_t* sorted,
-                                void* stream) {
+// separate: five launches whatever the device holds.
+int grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets, uint32_t* sorted, void* stream,
+                 bool separate) {
     if (n > MAX_BIRDS)
         return na_fail(FLK_ERR_CAPACITY, "flk_grid_noalloc: " + std::to_string(n) + " birds exceeds the maximum of " +
                                              std::to_string(MAX_BIRDS) + " this entry point's fixed scratch holds");
@@ -283,6 +302,8 @@ extern "C" int flk_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, u
     if (word) *(volatile uint32_t*)&g_status[(dev % STATUS_DEVICES) * 16] = 0;
     else if ((e = cudaMemsetAsync(s.ctl + CTL_ERROR, 0, 4, st)) != cudaSuccess)
         return na_fail(FLK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
+    uint32_t* status = word ? word : s.ctl + CTL_ERROR;
+    const float4* pos = reinterpret_cast<const float4*>(pos4);
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeCooperative;
     at.val.cooperative = 1;
@@ -290,20 +311,53 @@ extern "C" int flk_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, u
     cfg.gridDim = dim3(B / 2 / THREADS);  // 32 to 128 CTAs
     cfg.blockDim = dim3(THREADS);
     cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, k_na_grid, reinterpret_cast<const float4*>(pos4), n, B, keys, offsets, sorted, s,
-                           word ? word : s.ctl + CTL_ERROR);
-    if (e != cudaSuccess) return na_fail(FLK_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
+    const auto phases = [&] {
+        cfg.numAttrs = 0;
+        cudaError_t r = cudaSuccess;
+        for (uint32_t k = 0; k < PHASES && r == cudaSuccess; ++k)
+            r = cudaLaunchKernelEx(&cfg, k_na_grid<false>, pos, n, B, keys, offsets, sorted, s, status, k);
+        return r;
+    };
     uint32_t err = 0;
-    if (!word) e = cudaMemcpyAsync(&err, s.ctl + CTL_ERROR, 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return na_fail(FLK_ERR_CUDA, std::string("flk_grid_noalloc: ") + cudaGetErrorString(e));
-    if (word) err = *(volatile uint32_t*)&g_status[(dev % STATUS_DEVICES) * 16];
-    if (err == 1) {  // a barrier gave up: the next call finds it as after loading
-        cudaMemsetAsync(s.ctl, 0, SCRATCH_BYTES - OFF_CTL, st);
-        cudaStreamSynchronize(st);
+    // the error word once the stream is done
+    const auto finish = [&] {
+        err = 0;
+        cudaError_t r = word ? cudaSuccess : cudaMemcpyAsync(&err, status, 4, cudaMemcpyDeviceToHost, st);
+        if (r == cudaSuccess) r = cudaStreamSynchronize(st);
+        if (r == cudaSuccess && word) err = *(volatile uint32_t*)&g_status[(dev % STATUS_DEVICES) * 16];
+        return r;
+    };
+    if (!separate) {
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, k_na_grid<true>, pos, n, B, keys, offsets, sorted, s, status, 0u);
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+            (void)cudaGetLastError();
+            separate = true;
+        }
     }
+    if (separate) e = phases();
+    if (e != cudaSuccess) return na_fail(FLK_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
+    e = finish();
+    if (e == cudaSuccess && err == 1) {  // a barrier gave up: clear its counters, do without
+        if (word) *(volatile uint32_t*)&g_status[(dev % STATUS_DEVICES) * 16] = 0;
+        e = cudaMemsetAsync(s.ctl, 0, CTL_WORDS * 4, st);
+        if (e == cudaSuccess) e = phases();
+        if (e == cudaSuccess) e = finish();
+    }
+    if (e != cudaSuccess) return na_fail(FLK_ERR_CUDA, std::string("flk_grid_noalloc: ") + cudaGetErrorString(e));
     if (err) return na_fail(FLK_ERR_DEVICE, "flk_grid_noalloc: device error word " + std::to_string(err));
     return FLK_OK;
+}
+
+}  // namespace
+
+extern "C" int flk_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets, uint32_t* sorted,
+                                void* stream) {
+    return grid_noalloc(pos4, n, keys, offsets, sorted, stream, false);
+}
+
+extern "C" int flk_debug_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets,
+                                      uint32_t* sorted, void* stream, int32_t separate) {
+    return grid_noalloc(pos4, n, keys, offsets, sorted, stream, separate != 0);
 }
