@@ -314,9 +314,10 @@ void flk_host_free(void* ptr);
 #define FLK_NOALLOC_MAX_BIRDS 131072u
 int flk_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets, uint32_t* sorted, void* stream);
 /* Test hook: the same call by separate launches, as where the device cannot hold
- * the one kernel's blocks at once (`separate`). */
+ * the one kernel's blocks at once (`separate`), or one that leaves its barrier
+ * counters as calls that overlapped might (`spoil`). */
 int flk_debug_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets, uint32_t* sorted,
-                           void* stream, int32_t separate);
+                           void* stream, int32_t separate, int32_t spoil);
 
 #ifdef __cplusplus
 }

@@ -22,7 +22,8 @@
 // All calls share the one array and it keeps the previous call's contents:
 // each call clears the parts that must start at zero. Calls that overlap on the
 // GPU (different streams or threads, same device) race on the array and give
-// wrong results; serialise them.
+// wrong results; serialise them. Later calls are right again: a call's barrier
+// counters are its own (one of BARRIERS sets in turn, cleared half a turn before).
 //
 // A call is latency: at 131,072 birds three clears, four kernels and the error
 // word's copy took 49 us, of which the host's launches were nearly all. The
@@ -35,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 #include <string>
@@ -56,8 +58,9 @@ constexpr uint32_t FULL = 0xFFFFFFFFu;
 constexpr size_t OFF_COUNTS = 0;                                  // MAX_BUCKETS u32
 constexpr size_t OFF_TMP = OFF_COUNTS + MAX_BUCKETS * 4ull;       // MAX_BIRDS u32
 constexpr size_t OFF_CTL = OFF_TMP + MAX_BIRDS * 4ull;            // CTL_WORDS u32
-// an error; birds per tile; the barrier's counters (arrived, turns)
-enum { CTL_ERROR = 0, CTL_SUM = 64, CTL_BARRIER = 128, CTL_WORDS = CTL_BARRIER + 16 };
+constexpr uint32_t BARRIERS = 32;  // calls until a set of barrier counters is used again
+// an error; birds per tile; the barriers' counters (arrived, turns: 16 words a set)
+enum { CTL_ERROR = 0, CTL_SUM = 64, CTL_BARRIER = 128, CTL_WORDS = CTL_BARRIER + 16 * BARRIERS };
 enum { ARRIVED = 0, TURN = 8 };
 constexpr size_t SCRATCH_BYTES = OFF_CTL + CTL_WORDS * 4ull;
 constexpr int THREADS = 1024;        // per CTA
@@ -167,8 +170,8 @@ constexpr int PHASES = 5;  // clear, count, scan, scatter, order
 
 // buckets: a power of two of at least 2^16, and at least 2n; buckets / 2 threads.
 // *status: zero at the start, an error word where there was one.
-// FUSED: every phase (a cooperative launch); otherwise phase `arg` alone, the
-// arrival ranks waiting in `sorted` for the scatter.
+// FUSED: every phase, with barrier set `arg` (a cooperative launch); otherwise
+// phase `arg` alone, the arrival ranks waiting in `sorted` for the scatter.
 template <bool FUSED>
 __global__ void __launch_bounds__(THREADS, 1) k_na_grid(const float4* __restrict__ pos, uint32_t n, uint32_t buckets,
                                                         uint32_t* keys, uint32_t* offsets, uint32_t* sorted, Scratch s,
@@ -176,7 +179,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_na_grid(const float4* __restrict
     __shared__ uint32_t s_warp[THREADS / 32], s_tile[MAX_BUCKETS / TILE];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, v = blockIdx.x * THREADS + tid;
     const bool mine = v < n;  // this thread's bird
-    uint32_t* bar = s.ctl + CTL_BARRIER;
+    uint32_t* bar = s.ctl + CTL_BARRIER + 16 * arg;
     const auto runs = [&](uint32_t phase) { return FUSED || arg == phase; };
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t b = 0, arrival = 0;
@@ -185,6 +188,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_na_grid(const float4* __restrict
     if (runs(0)) {
         reinterpret_cast<uint2*>(s.counts)[v] = make_uint2(0u, 0u);
         if (v < MAX_BUCKETS / TILE) s.ctl[CTL_SUM + v] = 0;
+        if (FUSED && v < 16) s.ctl[CTL_BARRIER + 16 * ((arg + BARRIERS / 2) % BARRIERS) + v] = 0;
     }
     if (FUSED && !grid_barrier(bar, status)) return;
     // hash and count, each tile of buckets as a whole as well
@@ -273,9 +277,13 @@ int na_fail(int code, const std::string& m) {
     return code;
 }
 
-// separate: five launches whatever the device holds.
+// The last call's number on each device: which barrier counters the next one uses.
+std::atomic<uint32_t> g_calls[STATUS_DEVICES];
+
+// separate: five launches whatever the device holds; spoil: leaves the call's
+// barrier counters as calls that overlapped might.
 int grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets, uint32_t* sorted, void* stream,
-                 bool separate) {
+                 bool separate, bool spoil) {
     if (n > MAX_BIRDS)
         return na_fail(FLK_ERR_CAPACITY, "flk_grid_noalloc: " + std::to_string(n) + " birds exceeds the maximum of " +
                                              std::to_string(MAX_BIRDS) + " this entry point's fixed scratch holds");
@@ -311,9 +319,10 @@ int grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offset
     cfg.gridDim = dim3(B / 2 / THREADS);  // 32 to 128 CTAs
     cfg.blockDim = dim3(THREADS);
     cfg.stream = st;
+    const uint32_t set = g_calls[dev % STATUS_DEVICES].fetch_add(1) % BARRIERS;
     const auto phases = [&] {
         cfg.numAttrs = 0;
-        cudaError_t r = cudaSuccess;
+        cudaError_t r = cudaMemsetAsync(s.ctl + CTL_BARRIER + 16 * ((set + BARRIERS / 2) % BARRIERS), 0, 64, st);
         for (uint32_t k = 0; k < PHASES && r == cudaSuccess; ++k)
             r = cudaLaunchKernelEx(&cfg, k_na_grid<false>, pos, n, B, keys, offsets, sorted, s, status, k);
         return r;
@@ -330,7 +339,7 @@ int grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offset
     if (!separate) {
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, k_na_grid<true>, pos, n, B, keys, offsets, sorted, s, status, 0u);
+        e = cudaLaunchKernelEx(&cfg, k_na_grid<true>, pos, n, B, keys, offsets, sorted, s, status, set);
         if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
             (void)cudaGetLastError();
             separate = true;
@@ -345,6 +354,10 @@ int grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offset
         if (e == cudaSuccess) e = phases();
         if (e == cudaSuccess) e = finish();
     }
+    if (e == cudaSuccess && spoil) {
+        e = cudaMemsetAsync(s.ctl + CTL_BARRIER + 16 * set, 1, 16 * 4, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    }
     if (e != cudaSuccess) return na_fail(FLK_ERR_CUDA, std::string("flk_grid_noalloc: ") + cudaGetErrorString(e));
     if (err) return na_fail(FLK_ERR_DEVICE, "flk_grid_noalloc: device error word " + std::to_string(err));
     return FLK_OK;
@@ -354,10 +367,10 @@ int grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offset
 
 extern "C" int flk_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets, uint32_t* sorted,
                                 void* stream) {
-    return grid_noalloc(pos4, n, keys, offsets, sorted, stream, false);
+    return grid_noalloc(pos4, n, keys, offsets, sorted, stream, false, false);
 }
 
 extern "C" int flk_debug_grid_noalloc(const float* pos4, uint32_t n, uint32_t* keys, uint32_t* offsets,
-                                      uint32_t* sorted, void* stream, int32_t separate) {
-    return grid_noalloc(pos4, n, keys, offsets, sorted, stream, separate != 0);
+                                      uint32_t* sorted, void* stream, int32_t separate, int32_t spoil) {
+    return grid_noalloc(pos4, n, keys, offsets, sorted, stream, separate != 0, spoil != 0);
 }
