@@ -288,7 +288,8 @@ int flk_copies_straight(const void* ptr, uint64_t bytes);
 /* A page-locked buffer of at least `bytes` for results or states, from a
  * process-wide bounded cache, and its return to it (locking pages afresh costs
  * about a millisecond per 25 MB); safe from any thread. Private memory: a
- * forked child has its own copy. No counterpart. */
+ * forked child has its own copy. Callers hold at most 2 GiB of them at once
+ * (beyond that FLK_ERR_CUDA: use ordinary memory). No counterpart. */
 int flk_host_alloc(uint64_t bytes, void** ptr);
 void flk_host_free(void* ptr);
 

@@ -174,8 +174,9 @@ _LOCKED_MIN, _LOCKED_MAX = 8 << 10, 64 << 20
 
 
 def _result(n: int) -> np.ndarray:
-    """An uninitialised words array [n, 15], page-locked where that pays; its
-    block goes back to the library's cache with the last reference to it."""
+    """An uninitialised words array [n, 15], page-locked where that pays and
+    while the results held are below 2 GiB in all; its block goes back to the
+    library's cache with the last reference to it."""
     nbytes = n * WORDS * 4
     if _LOCKED_MIN <= nbytes <= _LOCKED_MAX:
         p = C.c_void_p()

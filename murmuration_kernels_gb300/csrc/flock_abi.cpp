@@ -1020,7 +1020,7 @@ extern "C" int flk_copies_straight(const void* ptr, uint64_t bytes) {
 extern "C" int flk_host_alloc(uint64_t bytes, void** ptr) {
     if (!ptr || !bytes) return fail(FLK_ERR_ARG, "flk_host_alloc: null pointer or zero size");
     return guarded([&] {
-        *ptr = flk::host_alloc((size_t)bytes);
+        *ptr = flk::host_alloc((size_t)bytes, true);
         return *ptr ? FLK_OK : fail(FLK_ERR_CUDA, "flk_host_alloc: no page-locked memory");
     });
 }

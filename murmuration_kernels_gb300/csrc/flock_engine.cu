@@ -198,13 +198,19 @@ void stream_put(int dev, cudaStream_t s) {
 // child would see its array change as the parent's next result takes the block
 // (both kinds copy at the link's rate: 1M birds read in 336 us, opened in 315).
 // Mapping and locking cost about a millisecond per 25 MB, so released blocks
-// wait here for the next of their size, at most HOST_CAP bytes of them.
-constexpr size_t HOST_CAP = 2ull << 30;
+// wait here for the next of their size, at most HOST_CAP bytes of them. Result
+// arrays that callers hold are page-locked up to RESULT_CAP bytes in all: a program
+// that keeps every frame must not lock the host's memory away.
+constexpr size_t HOST_CAP = 2ull << 30, RESULT_CAP = 2ull << 30;
 struct HostCache {
+    struct Block {
+        size_t bytes;
+        bool result;  // counted in `results`
+    };
     std::mutex mu;
     std::multimap<size_t, void*> free_blocks;
-    std::map<void*, size_t> sizes;
-    size_t cached = 0;
+    std::map<void*, Block> blocks;  // every block there is
+    size_t cached = 0, results = 0;
 };
 HostCache g_host;
 
@@ -235,31 +241,38 @@ cudaLaunchConfig_t small_config(uint32_t flocks, uint32_t ctas, uint32_t nmax, c
 }
 }  // namespace
 
-// A page-locked block of at least `bytes`, or null where the host gives none.
-// Sizes are rounded up to a quarter of their power of two (a page at least).
-void* host_alloc(size_t bytes) {
+// A page-locked block of at least `bytes`, or null where the host gives none or
+// (result) callers hold RESULT_CAP bytes of results. Sizes are rounded up to a
+// quarter of their power of two (a page at least).
+void* host_alloc(size_t bytes, bool result) {
     size_t unit = (size_t)sysconf(_SC_PAGESIZE);
     while (unit * 8 < bytes) unit *= 2;
     const size_t rb = std::max<size_t>(unit, (bytes + unit - 1) / unit * unit);
     {
         std::lock_guard<std::mutex> lk(g_host.mu);
+        if (result && g_host.results + rb > RESULT_CAP) return nullptr;
+        if (result) g_host.results += rb;
         auto it = g_host.free_blocks.find(rb);
         if (it != g_host.free_blocks.end()) {
             void* p = it->second;
             g_host.free_blocks.erase(it);
             g_host.cached -= rb;
+            g_host.blocks[p].result = result;
             return p;
         }
     }
     void* p = mmap(nullptr, rb, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_POPULATE, -1, 0);
-    if (p == MAP_FAILED) return nullptr;
-    if (cudaHostRegister(p, rb, cudaHostRegisterPortable | cudaHostRegisterMapped) != cudaSuccess) {
+    if (p != MAP_FAILED && cudaHostRegister(p, rb, cudaHostRegisterPortable | cudaHostRegisterMapped) != cudaSuccess) {
         (void)cudaGetLastError();
         munmap(p, rb);
-        return nullptr;
+        p = MAP_FAILED;
     }
     std::lock_guard<std::mutex> lk(g_host.mu);
-    g_host.sizes[p] = rb;
+    if (p == MAP_FAILED) {
+        if (result) g_host.results -= rb;
+        return nullptr;
+    }
+    g_host.blocks[p] = {rb, result};
     return p;
 }
 
@@ -267,16 +280,19 @@ void* host_alloc(size_t bytes) {
 void host_free(void* p) {
     if (!p) return;
     std::lock_guard<std::mutex> lk(g_host.mu);
-    auto it = g_host.sizes.find(p);
-    if (it == g_host.sizes.end()) return;
-    if (g_host.cached + it->second > HOST_CAP) {
+    auto it = g_host.blocks.find(p);
+    if (it == g_host.blocks.end()) return;
+    const size_t rb = it->second.bytes;
+    if (it->second.result) g_host.results -= rb;
+    it->second.result = false;
+    if (g_host.cached + rb > HOST_CAP) {
         if (cudaHostUnregister(p) != cudaSuccess) (void)cudaGetLastError();
-        munmap(p, it->second);
-        g_host.sizes.erase(it);
+        munmap(p, rb);
+        g_host.blocks.erase(it);
         return;
     }
-    g_host.free_blocks.emplace(it->second, p);
-    g_host.cached += it->second;
+    g_host.free_blocks.emplace(rb, p);
+    g_host.cached += rb;
 }
 
 template <class T>

@@ -321,7 +321,7 @@ uint32_t buckets_for(uint32_t n);
 uint32_t production_buckets(uint32_t n);
 
 // Page-locked host blocks from a bounded cache (null where the host gives none).
-void* host_alloc(size_t bytes);
+void* host_alloc(size_t bytes, bool result = false);
 void host_free(void* p);
 // Where kernels may access host memory [p, p + bytes) directly, or null.
 void* mapped(const void* p, size_t bytes);
