@@ -133,6 +133,9 @@ __device__ __forceinline__ float search_reach(f3 p, float r) {
     const float pm = fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z)));
     return rr * 1.00001f + 1e-3f + pm * 1e-6f;
 }
+// Radius above which a bird's box spans more than eight rows along y and z: 4 R (the
+// reach is at least 2 R to either side) is more than eight rows' width.
+inline float wide_radius(float cell) { return 8.01f * cell / ROWS_PER_CELL / 4.0f; }
 // The reference cells that reach touches.
 struct SearchBox {
     float reach, reach2;

@@ -1065,9 +1065,11 @@ void Engine::enqueue_step(bool sets, cudaEvent_t* ev, bool f64, bool hash, bool 
     if (ev) FLK_CUDA(cudaEventRecord(ev[2], stream_));
     k_scatter<<<sgrid(fit_.scatter), 256, 0, stream_>>>(table_d_, nfl, V_, ar_, key_, arrival_, offsets_, tmp_, ctl_);
     if (move)
-        k_order<true><<<sgrid(fit_.order[1]), 256, 0, stream_>>>(table_d_, nfl, V_, ctl_, tmp_, ar_, view_, due_);
+        k_order<true><<<sgrid(fit_.order[1]), 256, 0, stream_>>>(table_d_, nfl, V_, ctl_, tmp_, ar_, view_, due_,
+                                                                           wide_radius(cell));
     else
-        k_order<false><<<sgrid(fit_.order[0]), 256, 0, stream_>>>(table_d_, nfl, V_, ctl_, tmp_, ar_, view_, due_);
+        k_order<false><<<sgrid(fit_.order[0]), 256, 0, stream_>>>(table_d_, nfl, V_, ctl_, tmp_, ar_, view_, due_,
+                                                                           wide_radius(cell));
     if (f64) {  // FP64 evaluation from the input state, before the f32 passes change it
         k_decide_f64<<<pgrid(num_sms_, fit_.decide_f64, V_, 8), 256, 0, stream_>>>(table_d_, V_, ctl_, due_, offsets_, tile_end_, ar_,
                                                                                    dec64_, err64_, cell, inv_cell);

@@ -50,7 +50,7 @@ struct Arena {
 // block of the integrate pass), the scan epoch and the device error word.
 struct StepCtl {
     uint32_t due_count;    // deciding birds this step, from the list's start
-    uint32_t due_small;    // deciding birds of small flocks, from the list's end
+    uint32_t due_small;    // those of small flocks or with wide boxes, from the list's end
     uint32_t scan_ticket;  // dynamic tile ids of the scan
     uint32_t epoch;        // scan status tag, advanced once per step
     uint32_t done_blocks;  // integrate's last-block detector

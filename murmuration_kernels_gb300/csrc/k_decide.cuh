@@ -26,10 +26,10 @@
 // of dependent loads and operations: a whole warp per bird is the shortest one,
 // so flocks below SMALL_FLOCK birds are decided that way wherever they are
 // (alone or in a batch, so that a flock's result does not depend on it).
-// Birds with more than FAST_ROWS rows in their box, ROW_CAP non-empty ranges or
-// HIT_CAP hits in one lane are done by the whole warp, one at a time, after its
-// others; a box wider than the lattice or the flock sweeps the flock's whole
-// range.
+// Birds above wide_radius, in any flock, go the same way. Other birds with more than
+// FAST_ROWS rows in their box, ROW_CAP non-empty ranges or HIT_CAP hits in one lane
+// are done by the whole warp, one at a time, after its others; a box wider than the
+// lattice or the flock sweeps the flock's whole range.
 #pragma once
 
 #include "device_common.cuh"
@@ -46,6 +46,7 @@ constexpr uint32_t DECIDE_BATCH = 8;             // birds whose epilogues run to
 // Per-warp shared memory. It shares each SM's storage with the L1 cache that
 // holds the candidates, so it stays small.
 static_assert(ROW_CAP >= 32, "a warp that takes one bird lists 32 ranges at a time");
+static_assert(FAST_ROWS < 81, "wide_radius: more than eight rows along y and z are too many for a group");
 struct WarpSmem {
     uint2 row[DECIDE_GROUPS][ROW_CAP + 1];                // view ranges (padded against bank conflicts)
     uint32_t hit[DECIDE_GROUPS * HIT_CAP * DECIDE_LANES];  // places of hits, each group's part contiguous
@@ -649,8 +650,8 @@ __device__ __noinline__ uint2 warp_bird(WarpSmem& m, const DueRec* __restrict__ 
     return make_uint2(cand, a.n_g);
 }
 
-// The birds of small flocks (their records fill the list from its end), one per
-// warp, spread over the CTAs.
+// The birds of small flocks and those with a radius above wide_radius (their records
+// fill the list from its end), one per warp, spread over the CTAs.
 __device__ __forceinline__ void small_birds(WarpSmem& m, uint32_t V, uint32_t nsmall, const DueRec* __restrict__ due,
                                             const FlockDesc* __restrict__ fl, StepCtl* __restrict__ ctl,
                                             const uint32_t* __restrict__ offsets,

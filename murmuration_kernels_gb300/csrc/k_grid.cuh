@@ -432,6 +432,12 @@ __global__ void __launch_bounds__(256) k_scatter(const FlockDesc* __restrict__ f
 // ranks are counted, so that neighbours in the list are neighbours in space and
 // the list follows the order within the chip's window (longer contiguous parts
 // per CTA spread the list over the flock: decide 1.08 -> 1.28 ms at 16.7M birds).
+// Decide takes the records of one list by groups of eight lanes and those of the
+// other by whole warps, spread over the chip: the birds of small flocks, and birds
+// whose radius alone makes their box too wide for a group (wide_radius; NaN too),
+// which a group would only mark and its warp come back to, one after the other
+// (9,000 birds a hundred times thinner than the benchmark's, radius 7 m, 132 -> 67
+// us a step, 1M of them 768 -> 733; dense flocks the same, 1M 128).
 // MOVE: the state moves into the flock's other buffer in the new order as well.
 // Birds change their neighbourhood slowly (5 cm a step), so the slots of a
 // recent order still give mostly contiguous gathers, and most steps leave the
@@ -444,7 +450,8 @@ __global__ void __launch_bounds__(256) k_scatter(const FlockDesc* __restrict__ f
 template <bool MOVE>
 __global__ void __launch_bounds__(256, MOVE ? 5 : 8) k_order(const FlockDesc* __restrict__ fl, int nfl, uint32_t V,
                                                StepCtl* __restrict__ ctl, const uint2* __restrict__ tmp, Arena ar,
-                                               float4* __restrict__ view, DueRec* __restrict__ due) {
+                                               float4* __restrict__ view, DueRec* __restrict__ due,
+                                               float wide_radius) {
     __shared__ uint32_t s_cnt[2][8];
     __shared__ uint2 s_base[2];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -475,6 +482,7 @@ __global__ void __launch_bounds__(256, MOVE ? 5 : 8) k_order(const FlockDesc* __
                         c = ar.C[st];
                         next = ar.next[st];
                     }
+                    if (is_due) small = small || !(c.w <= wide_radius);
                     if (MOVE) e = ar.D[st];
                 } else {  // never with a consistent grid
                     f = -1;
@@ -484,7 +492,7 @@ __global__ void __launch_bounds__(256, MOVE ? 5 : 8) k_order(const FlockDesc* __
                 f = -1;
             }
         }
-        // two lists: records from the start, small flocks' from the end; the
+        // two lists: groups' records from the start, warps' from the end; the
         // counts of both ride in one word (256 records at most)
         const uint32_t dm = __ballot_sync(FULL, is_due && !small), ds = __ballot_sync(FULL, is_due && small);
         if (lane == 0) s_cnt[it][warp] = __popc(dm) | (uint32_t)__popc(ds) << 16;
