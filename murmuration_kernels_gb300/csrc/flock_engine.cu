@@ -1215,10 +1215,14 @@ void Engine::launch_graph(const StepGraph& sg) {
 // A kernel launch takes the host about 7 us, a graph launch no more, and a
 // mid-size step's five kernels 28 us on the GPU: launched one by one they keep it
 // waiting (37,501 birds: 38 us a step against 29 in graphs). A step graph is
-// cheap to capture (five nodes), so any run of a few steps goes through it; a
-// graph of a whole chunk (a few percent faster still) is built for long runs and
-// for handles that run again and again, while the GPU is busy with the first
-// chunk. The launches are the captured ones, so the results are the same.
+// cheap to capture (five nodes), so any run of a few steps goes through it. A
+// graph of a whole chunk has no gap between its steps (us a step, step graphs
+// against chunk graphs: 8,193 birds 26.0 / 23.7, 37,501 29.6 / 26.3, 100,000
+// 31.7 / 27.7, 300,000 45.6 / 42.7, 1M 109 / 105); it is built for runs of ten
+// chunks and for the third run of a table that stays the same, a served pool's
+// chunks among them (its median latency under a Poisson load 14.8 -> 13.5 ms),
+// while the GPU is busy with a chunk. The launches are the captured ones, so the
+// results are the same.
 void Engine::enqueue_run(uint32_t steps) {
     if (const uint32_t ctas = small_ctas()) {
         enqueue_small(steps, ctas);
@@ -1229,7 +1233,7 @@ void Engine::enqueue_run(uint32_t steps) {
     uint32_t done = 0;
     if (steps >= chunk) {
         const bool ready = chunk_graph_.exec && chunk_graph_.steps == chunk && !chunk_graph_.stale;
-        if (ready || steps >= 10 * chunk || (same_runs_ >= 2 && steps >= 2 * chunk)) {
+        if (ready || steps >= 10 * chunk || same_runs_ >= 2) {
             if (!ready) {
                 enqueue_singly(chunk);
                 done = chunk;
