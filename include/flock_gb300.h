@@ -165,9 +165,15 @@ int flk_batch_tune_cell(flk_batch* b, float cell_m);
  * values: FLK_ERR_ARG. No counterpart: the reference's decide
  * (cuda/flock.cu:190-290) reads every candidate from global memory. */
 int flk_batch_tune_decide(flk_batch* b, int32_t staged);
-/* Chunk graphs instantiated, and updated in place (cudaGraphExecUpdate, when
- * only sizes or pointers changed, e.g. a flock joined or left), so far. */
+/* Graphs (of one step, and of a chunk of steps) instantiated, and updated in place
+ * (cudaGraphExecUpdate, when only sizes or pointers changed, e.g. a flock joined
+ * or left), so far. */
 int flk_batch_graph_counts(flk_batch* b, uint64_t* instantiated, uint64_t* updated);
+/* How flk_batch_step runs the batch as it is: *ctas thread blocks per flock, one
+ * cluster each, in one kernel for all steps (every flock is small and all the
+ * clusters fit on the GPU; the launch shapes above have no effect then), or 0,
+ * one kernel per pass. The same results either way. */
+int flk_batch_small_ctas(flk_batch* b, uint32_t* ctas);
 /* flk_counters summed over the batch's flocks. */
 int flk_batch_counters(flk_batch* b, uint64_t* due, uint64_t* candidates, uint64_t* pairs);
 /* Times `steps` graph-launched steps on the batch's stream with CUDA events. */

@@ -119,6 +119,7 @@ _SIGS = {
     "flk_kernels_per_step": (C.c_int, []),
     "flk_pin": (C.c_int, [C.c_void_p, C.c_uint64]),
     "flk_unpin": (C.c_int, [C.c_void_p]),
+    "flk_batch_small_ctas": (C.c_int, [_P, C.POINTER(C.c_uint32)]),
     "flk_copies_straight": (C.c_int, [C.c_void_p, C.c_uint64]),
     "flk_host_alloc": (C.c_int, [C.c_uint64, C.POINTER(C.c_void_p)]),
     "flk_host_free": (None, [C.c_void_p]),
@@ -457,10 +458,17 @@ class Batch:
         return res
 
     def graph_counts(self) -> tuple[int, int]:
-        """(chunk graphs instantiated, chunk graphs updated in place) so far."""
+        """(graphs instantiated, graphs updated in place) so far, of one step or a chunk."""
         a, b = C.c_uint64(), C.c_uint64()
         _check(lib().flk_batch_graph_counts(self._h, C.byref(a), C.byref(b)))
         return a.value, b.value
+
+    def small_ctas(self) -> int:
+        """Thread blocks per flock where step() runs the batch as one cluster per
+        flock in one kernel, 0 where it runs one kernel per pass."""
+        k = C.c_uint32()
+        _check(lib().flk_batch_small_ctas(self._h, C.byref(k)))
+        return k.value
 
     def tune(self, stream_bps: int = 0, decide_bps: int = 0, decide_threads: int = 0, graph_chunk: int = 0,
              cell: float = 0.0, staged: int = -1) -> None:

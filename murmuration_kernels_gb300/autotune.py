@@ -7,11 +7,16 @@ steps captured per CUDA graph. The production steps' cell edge is one too
 (`cell`, in metres; birds are sorted into rows of buckets a sixth of it along
 x and 2/3 of it along y and z): a smaller cell means fewer candidates per
 deciding bird but more rows per search box, and more buckets. Any edge finds
-the same neighbours. Clusters are not used, so there is no cluster shape to tune. The best values depend on the workload (one
+the same neighbours. The best values depend on the workload (one
 1M-bird flock vs hundreds of small flocks), so the tuner measures them on the
 actual batch: coordinate descent over each knob's candidate values, each
 candidate timed with CUDA events over a few graph-launched steps, keeping a
 change only when it beats the incumbent by more than the noise margin.
+
+A batch of small flocks runs as one thread-block cluster per flock
+(`Batch.small_ctas`); the cluster's size follows from the number and the sizes of
+the flocks and is not tuned, and of the knobs above only the cell has an effect,
+so only it is tried there.
 
 Results are cached per (GPU name, workload signature) in a JSON file so a
 served or batched run can reuse them:
@@ -84,7 +89,10 @@ def tune(batch, steps: int = 10, reps: int = 2, margin: float = 0.01, gpu: str =
     best = dict(DEFAULT)
     best_t = _time(batch, best, steps, reps)
     trials = 1
+    clusters = getattr(batch, "small_ctas", lambda: 0)()
     for knob, values in SPACE.items():
+        if clusters and knob != "cell":
+            continue  # no effect: what it timed would be noise
         start = best[knob]  # timed already, as part of the incumbent
         for v in values:
             if v == start or v == best[knob]:

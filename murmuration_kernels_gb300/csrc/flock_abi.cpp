@@ -456,6 +456,14 @@ extern "C" int flk_batch_graph_counts(flk_batch* b, uint64_t* instantiated, uint
     return FLK_OK;
 }
 
+extern "C" int flk_batch_small_ctas(flk_batch* b, uint32_t* ctas) {
+    if (!b || !ctas) return fail(FLK_ERR_ARG, "flk_batch_small_ctas: null pointer");
+    return guarded([&] {
+        *ctas = b->eng->small_ctas_of_all();
+        return FLK_OK;
+    });
+}
+
 extern "C" int flk_batch_counters(flk_batch* b, uint64_t* due, uint64_t* cand, uint64_t* pairs) {
     if (!b) return fail(FLK_ERR_ARG, "flk_batch_counters: null handle");
     return guarded([&] {

@@ -1130,17 +1130,28 @@ void Engine::enqueue_steps(uint32_t n) {
 // 9.7 / 21.1, of 4,000 20.7 / 26.2; 18 flocks (8) of 1,000 11.6 / 22.6, of 4,000
 // 32 / 32; 20 flocks (4) of 2,000 18.8 / 28.3; 37 flocks (2) of 1,000 17.2 / 27.5;
 // 150 flocks (1) of 500 15.9 / 33.9. Clusters in a second turn take as long again.
-uint32_t Engine::small_ctas() const {
-    if (shape_.decide_kind != 0 || table_h_.empty()) return 0;
-    uint32_t nmax = 0;
-    for (const FlockDesc& d : table_h_) nmax = std::max(nmax, d.n);
+uint32_t Engine::small_ctas(size_t flocks, uint32_t nmax) const {
+    if (shape_.decide_kind != 0 || !flocks) return 0;
     for (int k = 0; k < SMALL_SIZES; ++k) {
         const uint32_t ctas = SMALL_CTAS >> k;
         if (nmax <= std::min(SMALL_CLUSTER, ctas * SMALL_THREADS) &&
-            (int)table_h_.size() <= g_static[device_ % CACHE_DEVICES].small_clusters[k])
+            (int)flocks <= g_static[device_ % CACHE_DEVICES].small_clusters[k])
             return ctas;
     }
     return 0;
+}
+
+uint32_t Engine::small_ctas() const {
+    uint32_t nmax = 0;
+    for (const FlockDesc& d : table_h_) nmax = std::max(nmax, d.n);
+    return small_ctas(table_h_.size(), nmax);
+}
+
+uint32_t Engine::small_ctas_of_all() const {
+    uint32_t nmax = 0;
+    const std::vector<int> ids = flock_ids();
+    for (int id : ids) nmax = std::max(nmax, flock_size(id));
+    return small_ctas(ids.size(), nmax);
 }
 
 // A launch runs at most SMALL_STEPS steps, 0.1 s or so.

@@ -184,6 +184,9 @@ public:
     size_t device_bytes() const { return dev_bytes_; }
     // Cumulative counters from the step-control block.
     void counters(unsigned long long* due, unsigned long long* cand, unsigned long long* pairs);
+    // How a step of all resident flocks runs: CTAs per flock in one kernel of a
+    // cluster each, or 0 for the separate kernels.
+    uint32_t small_ctas_of_all() const;
     // Graphs instantiated, and updated in place, so far.
     void graph_counts(uint64_t* instantiated, uint64_t* updated) const {
         *instantiated = graph_instantiations_;
@@ -223,6 +226,7 @@ private:
     // first step counts its own, the last one counts none).
     void enqueue_steps(uint32_t n);
     // `steps` steps of a table of small flocks, a cluster each.
+    uint32_t small_ctas(size_t flocks, uint32_t nmax) const;
     uint32_t small_ctas() const;
     int pick_decide() const;
     void enqueue_small(uint32_t steps, uint32_t ctas);
