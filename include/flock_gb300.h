@@ -298,6 +298,9 @@ int flk_copies_straight(const void* ptr, uint64_t bytes);
  * (beyond that FLK_ERR_CUDA: use ordinary memory). No counterpart. */
 int flk_host_alloc(uint64_t bytes, void** ptr);
 void flk_host_free(void* ptr);
+/* Test hook: the calling thread's next `count` requests for page-locked memory
+ * fail, as on a host that locks no more. Everything runs without it. */
+int flk_debug_fail_locks(uint32_t count);
 
 /* ---- grid build without device allocation ------------------------------- */
 /* No counterpart in the reference. For callers that may not allocate device

@@ -120,6 +120,7 @@ _SIGS = {
     "flk_pin": (C.c_int, [C.c_void_p, C.c_uint64]),
     "flk_unpin": (C.c_int, [C.c_void_p]),
     "flk_batch_small_ctas": (C.c_int, [_P, C.POINTER(C.c_uint32)]),
+    "flk_debug_fail_locks": (C.c_int, [C.c_uint32]),
     "flk_copies_straight": (C.c_int, [C.c_void_p, C.c_uint64]),
     "flk_host_alloc": (C.c_int, [C.c_uint64, C.POINTER(C.c_void_p)]),
     "flk_host_free": (None, [C.c_void_p]),

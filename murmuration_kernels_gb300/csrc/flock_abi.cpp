@@ -1017,6 +1017,11 @@ extern "C" int flk_unpin(void* ptr) {
     return FLK_OK;
 }
 
+extern "C" int flk_debug_fail_locks(uint32_t count) {
+    flk::fail_locks(count);
+    return FLK_OK;
+}
+
 extern "C" int flk_copies_straight(const void* ptr, uint64_t bytes) {
     try {
         return flk::mapped(ptr, (size_t)bytes) != nullptr;

@@ -45,6 +45,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -241,10 +242,14 @@ cudaLaunchConfig_t small_config(uint32_t flocks, uint32_t ctas, uint32_t nmax, c
 }
 }  // namespace
 
+static thread_local uint32_t t_fail_locks = 0;  // test hook: host_alloc calls of this thread that still fail
+void fail_locks(uint32_t count) { t_fail_locks = count; }
+
 // A page-locked block of at least `bytes`, or null where the host gives none or
 // (result) callers hold RESULT_CAP bytes of results. Sizes are rounded up to a
 // quarter of their power of two (a page at least).
 void* host_alloc(size_t bytes, bool result) {
+    if (t_fail_locks) return --t_fail_locks, nullptr;
     size_t unit = (size_t)sysconf(_SC_PAGESIZE);
     while (unit * 8 < bytes) unit *= 2;
     const size_t rb = std::max<size_t>(unit, (bytes + unit - 1) / unit * unit);
@@ -276,12 +281,13 @@ void* host_alloc(size_t bytes, bool result) {
     return p;
 }
 
-// Gives a block of host_alloc back (no copy in flight may use it).
-void host_free(void* p) {
-    if (!p) return;
+// Gives a block of host_alloc back (no copy in flight may use it). False where p is
+// none.
+bool host_free(void* p) {
+    if (!p) return false;
     std::lock_guard<std::mutex> lk(g_host.mu);
     auto it = g_host.blocks.find(p);
-    if (it == g_host.blocks.end()) return;
+    if (it == g_host.blocks.end()) return false;
     const size_t rb = it->second.bytes;
     if (it->second.result) g_host.results -= rb;
     it->second.result = false;
@@ -289,10 +295,23 @@ void host_free(void* p) {
         if (cudaHostUnregister(p) != cudaSuccess) (void)cudaGetLastError();
         munmap(p, rb);
         g_host.blocks.erase(it);
-        return;
+        return true;
     }
     g_host.free_blocks.emplace(rb, p);
     g_host.cached += rb;
+    return true;
+}
+
+// An engine's control block: page-locked, or ordinary memory where the host locks
+// no more (its copies then return when they are done).
+static uint8_t* control_alloc(size_t bytes) {
+    void* p = host_alloc(bytes);
+    if (!p && !(p = std::malloc(bytes))) throw Error{-3, "host allocation failed"};
+    return static_cast<uint8_t*>(p);
+}
+static void control_free(uint8_t*& p) {
+    if (!host_free(p)) std::free(p);
+    p = nullptr;
 }
 
 template <class T>
@@ -401,8 +420,8 @@ Engine::~Engine() {
     dfree(view_); dfree(counts_); dfree(offsets_); dfree(tile_end_); dfree(even_);
     dfree(status_); dfree(sets_);
     dfree(block_); dfree(staging_); dfree(inv_);
-    host_free(h_up_);
-    host_free(h_down_);
+    control_free(h_up_);
+    control_free(h_down_);
     dfree(dec64_); dfree(out64_); dfree(active_); dfree(err64_);
     stream_put(device_, copy_);
     stream_put(device_, stream_);
@@ -616,7 +635,7 @@ std::vector<int> Engine::flock_ids() const {
 // page-locked host block each way, so that a call waits for the GPU once: the
 // steps, then one copy of the error word, clocks and countdowns.
 void Engine::ensure_block(uint32_t flocks) {
-    if (block_ && flocks <= table_cap_) return;
+    if (h_down_ && flocks <= table_cap_) return;
     const uint32_t cap = std::max(flocks, table_cap_ * 2);
     const size_t bytes = BLOCK_TABLE + (size_t)cap * sizeof(FlockDesc);
     size_t acct = 0;
@@ -630,11 +649,10 @@ void Engine::ensure_block(uint32_t flocks) {
     table_d_ = reinterpret_cast<FlockDesc*>(block_ + BLOCK_TABLE);
     table_cap_ = cap;
     FLK_CUDA(cudaStreamSynchronize(stream_));  // the last upload has left its host block
-    host_free(h_up_);
-    host_free(h_down_);
-    h_up_ = static_cast<uint8_t*>(host_alloc(bytes));
-    h_down_ = static_cast<uint8_t*>(host_alloc(bytes));
-    if (!h_up_ || !h_down_) throw Error{-3, "page-locked host allocation failed"};
+    control_free(h_up_);
+    control_free(h_down_);
+    h_up_ = control_alloc(bytes);
+    h_down_ = control_alloc(bytes);
     ctl_seen_ = false;
     free_graphs();
 }

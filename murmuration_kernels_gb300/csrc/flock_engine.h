@@ -326,7 +326,8 @@ uint32_t production_buckets(uint32_t n);
 
 // Page-locked host blocks from a bounded cache (null where the host gives none).
 void* host_alloc(size_t bytes, bool result = false);
-void host_free(void* p);
+bool host_free(void* p);
+void fail_locks(uint32_t count);  // test hook: the calling thread's next host_alloc calls fail
 // Where kernels may access host memory [p, p + bytes) directly, or null.
 void* mapped(const void* p, size_t bytes);
 
