@@ -481,15 +481,25 @@ size_t Engine::decide_smem(bool sets) const {
     return std::max(own, std::min(own + shape_.decide_extra_smem, smem_optin_));
 }
 
+// k_decide with `threads` picked by the engine (pick_decide) or the caller's (0).
+static auto decide_kernel(int threads) {
+    return threads == DECIDE_FEW ? k_decide<DECIDE_FEW> : threads == DECIDE_SOME ? k_decide<DECIDE_SOME>
+                                                                                 : k_decide<DECIDE_MANY>;
+}
+
 void Engine::decide_occupancy(int* blocks_per_sm, int* threads, size_t* smem_bytes) const {
-    const size_t smem = decide_smem(false);
+    std::vector<uint32_t> sizes;
+    for (int id : flock_ids()) sizes.push_back(flock_size(id));
+    const int picked = pick_decide(sizes);
+    const size_t smem = picked ? decide_bytes(picked) : decide_smem(false);
+    const int t = picked ? picked : shape_.decide_threads;
     int n = 0;
     if (shape_.decide_kind == 1)
-        FLK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_decide_staged, shape_.decide_threads, smem));
+        FLK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_decide_staged, t, smem));
     else
-        FLK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_decide<DECIDE_MANY>, shape_.decide_threads, smem));
+        FLK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decide_kernel(picked), t, smem));
     *blocks_per_sm = n;
-    *threads = shape_.decide_threads;
+    *threads = t;
     *smem_bytes = smem;
 }
 
@@ -1010,12 +1020,17 @@ void Engine::rebuild_table(bool grid_output) {
 // 105, 32 110; 8M: 28 727, 32 727; 16.7M: 28 1,525, 32 1,512. A caller's own launch
 // shape is used as it is (0).
 int Engine::pick_decide() const {
+    std::vector<uint32_t> sizes;
+    for (const FlockDesc& d : table_h_) sizes.push_back(d.n);
+    return pick_decide(sizes);
+}
+int Engine::pick_decide(const std::vector<uint32_t>& sizes) const {
     const LaunchShape own;
     if (shape_.decide_kind != own.decide_kind || shape_.decide_threads != own.decide_threads ||
         shape_.decide_blocks_per_sm != own.decide_blocks_per_sm || shape_.decide_extra_smem != own.decide_extra_smem)
         return 0;
     uint64_t birds = 0;  // four per warp
-    for (const FlockDesc& d : table_h_) birds += d.n < SMALL_FLOCK ? (uint64_t)d.n * DECIDE_GROUPS : d.n;
+    for (uint32_t n : sizes) birds += n < SMALL_FLOCK ? (uint64_t)n * DECIDE_GROUPS : n;
     const auto turn = [&](int threads) { return (uint64_t)num_sms_ * (threads / 32) * DECIDE_GROUPS * 10; };
     return birds <= 2 * turn(DECIDE_FEW) ? DECIDE_FEW : birds <= 50 * turn(DECIDE_SOME) ? DECIDE_SOME : DECIDE_MANY;
 }
@@ -1103,10 +1118,7 @@ void Engine::enqueue_step(bool sets, cudaEvent_t* ev, bool f64, bool hash, bool 
         k_decide_staged<<<dblocks, dthreads, decide_smem(false), stream_>>>(
             table_d_, V_, ctl_, due_, offsets_, tile_end_, ar_, view_, radius_table_, cell, inv_cell, STAGE_CAP);
     } else {
-        const auto kernel = decide_threads_ == DECIDE_FEW    ? k_decide<DECIDE_FEW>
-                            : decide_threads_ == DECIDE_SOME ? k_decide<DECIDE_SOME>
-                                                             : k_decide<DECIDE_MANY>;
-        kernel<<<dblocks, dthreads, decide_threads_ ? decide_bytes(dthreads) : decide_smem(false), stream_>>>(
+        decide_kernel(decide_threads_)<<<dblocks, dthreads, decide_threads_ ? decide_bytes(dthreads) : decide_smem(false), stream_>>>(
             table_d_, V_, ctl_, due_, offsets_, tile_end_, ar_, view_, radius_table_, cell, inv_cell);
     }
     if (ev) FLK_CUDA(cudaEventRecord(ev[4], stream_));

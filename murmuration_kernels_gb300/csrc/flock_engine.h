@@ -176,8 +176,8 @@ public:
     int num_sms() const { return num_sms_; }
     LaunchShape& shape() { return shape_; }
     void set_shape(const LaunchShape& s);
-    // decide's launch as configured: resident CTAs per SM, threads per CTA and
-    // dynamic shared memory per CTA (bytes), for production steps
+    // decide's launch in production steps of all resident flocks: resident CTAs per
+    // SM, threads per CTA and dynamic shared memory per CTA (bytes)
     void decide_occupancy(int* blocks_per_sm, int* threads, size_t* smem_bytes) const;
     // decide's dynamic shared memory per CTA for a step kind (its own + the reserved extra)
     size_t decide_smem(bool sets) const;
@@ -228,7 +228,8 @@ private:
     // `steps` steps of a table of small flocks, a cluster each.
     uint32_t small_ctas(size_t flocks, uint32_t nmax) const;
     uint32_t small_ctas() const;
-    int pick_decide() const;
+    int pick_decide() const;  // of the table
+    int pick_decide(const std::vector<uint32_t>& sizes) const;
     void enqueue_small(uint32_t steps, uint32_t ctas);
     // The production hash and count of the current positions.
     void enqueue_hash();
