@@ -175,6 +175,13 @@ def _words(words: np.ndarray) -> np.ndarray:
 _LOCKED_MIN, _LOCKED_MAX = 8 << 10, 64 << 20
 
 
+def _give_back(ptr: int, pid: int) -> None:
+    # a forked child only has a copy, and of the cache's lock as well, which another
+    # thread of the parent may have held
+    if os.getpid() == pid:
+        lib().flk_host_free(ptr)
+
+
 def _result(n: int) -> np.ndarray:
     """An uninitialised words array [n, 15], page-locked where that pays and
     while the results held are below 2 GiB in all; its block goes back to the
@@ -184,7 +191,7 @@ def _result(n: int) -> np.ndarray:
         p = C.c_void_p()
         if lib().flk_host_alloc(nbytes, C.byref(p)) == FLK_OK:
             block = (C.c_char * nbytes).from_address(p.value)
-            weakref.finalize(block, lib().flk_host_free, p.value).atexit = False
+            weakref.finalize(block, _give_back, p.value, os.getpid()).atexit = False
             return np.frombuffer(block, dtype=np.float32).reshape(n, WORDS)
     return np.empty((n, WORDS), dtype=np.float32)
 

@@ -38,3 +38,21 @@ def test_a_forked_child_keeps_its_array(native, n):
     assert w.ctypes.data == at and status == 0
     assert w.tobytes() == want == f.read()[1].tobytes()
     f.close()
+
+
+def test_a_child_gives_no_block_back(native, monkeypatch):
+    f = native.Flock(native.generate(2000, 2))
+    w = f.read()[1]
+    returned = []
+    monkeypatch.setattr(native.lib(), "flk_host_free", returned.append, raising=False)
+    pid = os.fork()
+    if pid == 0:
+        del w
+        os._exit(len(returned))
+    _, status = os.waitpid(pid, 0)
+    assert status == 0 and not returned
+    del w  # the parent's goes back
+    assert len(returned) == 1
+    monkeypatch.undo()
+    native.lib().flk_host_free(returned[0])
+    f.close()
