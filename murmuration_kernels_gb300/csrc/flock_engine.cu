@@ -333,13 +333,14 @@ void Engine::dfree(T*& p) {
     p = nullptr;
 }
 
-// The device address of host memory [p, p + bytes) that lies in one page-locked
-// range, or null: where it is not page-locked, only part of it is (two
-// registrations may lie within it and pages between them that a kernel must not
-// touch; device addresses equal host addresses, so the ends alone do not tell),
-// or the kernels' 4-byte words would not be aligned (a float32 view at an odd byte
-// offset: the copy engine takes any address, a load or store does not).
-void* mapped(const void* p, size_t bytes) {
+// What CUDA knows of the memory at p: nothing of ordinary host memory (type 0).
+namespace {
+struct Known {
+    unsigned int type = 0, managed = 0;
+    unsigned long long at = 0, start = 0;  // device address; start and size of its range
+    size_t size = 0;
+};
+Known known(const void* p) {
     using Query = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
     static const Query query = [] {
         void* f = nullptr;
@@ -351,19 +352,32 @@ void* mapped(const void* p, size_t bytes) {
         }
         return reinterpret_cast<Query>(f);
     }();
-    if (!query || reinterpret_cast<uintptr_t>(p) % sizeof(float)) return nullptr;
-    unsigned int type = 0, managed = 0;
-    unsigned long long at = 0, start = 0;
-    size_t size = 0;
+    Known k;
     CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
                                   CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
-    void* to[] = {&type, &managed, &at, &start, &size};
-    if (query(5, what, to, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return nullptr;
-    if (type != CU_MEMORYTYPE_HOST || managed || !at || at < start) return nullptr;
-    const size_t before = (size_t)(at - start);
-    return before < size && bytes <= size - before ? reinterpret_cast<void*>((uintptr_t)at) : nullptr;
+    void* to[] = {&k.type, &k.managed, &k.at, &k.start, &k.size};
+    if (!query || query(5, what, to, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) {
+        k = Known{};
+        k.type = ~0u;  // not known to be ordinary either
+    }
+    return k;
 }
+}  // namespace
+
+// The device address of host memory [p, p + bytes) that lies in one page-locked
+// range, or null: where it is not page-locked, only part of it is (two
+// registrations may lie within it and pages between them that a kernel must not
+// touch; device addresses equal host addresses, so the ends alone do not tell),
+// or the kernels' 4-byte words would not be aligned (a float32 view at an odd byte
+// offset: the copy engine takes any address, a load or store does not).
+static void* mapped(const Known& k, const void* p, size_t bytes) {
+    if (reinterpret_cast<uintptr_t>(p) % sizeof(float)) return nullptr;
+    if (k.type != CU_MEMORYTYPE_HOST || k.managed || !k.at || k.at < k.start) return nullptr;
+    const size_t before = (size_t)(k.at - k.start);
+    return before < k.size && bytes <= k.size - before ? reinterpret_cast<void*>((uintptr_t)k.at) : nullptr;
+}
+void* mapped(const void* p, size_t bytes) { return mapped(known(p), p, bytes); }
 
 Engine::Engine(int device) {
     if (device < 0) FLK_CUDA(cudaGetDevice(&device));
@@ -601,7 +615,8 @@ int Engine::add_flock(uint32_t n, float time, const float* words) {
                        free_ranges_.end());
     if (n) {
         const size_t bytes = (size_t)n * WORDS * 4;
-        const float* src = static_cast<const float*>(mapped(words, bytes));
+        const Known at = known(words);
+        const float* src = static_cast<const float*>(mapped(at, words, bytes));
         if (!src) {  // by way of a staging copy
             ensure_staging(bytes);
             FLK_CUDA(cudaMemcpyAsync(staging_, words, bytes, cudaMemcpyHostToDevice, stream_));
@@ -609,9 +624,12 @@ int Engine::add_flock(uint32_t n, float time, const float* words) {
         }
         k_unpack<<<pack_blocks(n), PACK_WARPS * 32, 0, stream_>>>(src, n, sbase, ar_);  // buffer 0
         FLK_CUDA(cudaGetLastError());
-        // page-locked words are read after the launches return: the caller may
-        // change them, or give their memory back, as soon as this call does
-        FLK_CUDA(cudaStreamSynchronize(stream_));
+        // Page-locked words are read after the launches return: the caller may
+        // change them, or give their memory back, as soon as this call does.
+        // Ordinary memory has been staged by then (200 flocks of 300 birds added in
+        // 4.4 ms with a wait each, 2.5 without).
+        if (at.type || known(reinterpret_cast<const char*>(words) + bytes - 1).type)
+            FLK_CUDA(cudaStreamSynchronize(stream_));
     }
     Slot s;
     s.n = n;
