@@ -212,6 +212,7 @@ private:
     };
     void ensure_arena(uint32_t need);
     void ensure_staging(size_t bytes);
+    bool bounce_block();
     int pack_blocks(uint32_t n) const;
     void enqueue_pack(float* dst, const Slot& s, uint32_t* inv);
     void rebuild_table(bool grid_output);
@@ -280,6 +281,8 @@ private:
     // blocks its contents go out from and come back to
     static constexpr size_t BLOCK_TABLE = 256;
     uint8_t *block_ = nullptr, *h_up_ = nullptr, *h_down_ = nullptr;
+    uint8_t* h_bounce_ = nullptr;   // bounce_block, and its device address
+    float* bounce_at_ = nullptr;
     bool ctl_seen_ = false;   // h_down_ holds the control block after all work so far
     bool uploading_ = false;  // a copy from h_up_ may be in flight
     bool idle_ = false;       // the engine is being destroyed and its streams are idle
