@@ -171,8 +171,10 @@ def _words(words: np.ndarray) -> np.ndarray:
 # Result arrays in page-locked memory: the state crosses the link straight into
 # them, and a fresh pageable array would cost its page faults as well (24 flocks
 # of 0.9 M birds read back in 3.2 ms). Outside this range the lock or the
-# bookkeeping costs more than it gives.
-_LOCKED_MIN, _LOCKED_MAX = 8 << 10, 64 << 20
+# bookkeeping costs more than it gives (us for a read into a page-locked array, and
+# into an ordinary one by way of the engine's block: 500 birds 20.7 / 18.6, 1,000
+# 20.4 / 20.0, 1,400 20.3 / 21.3, 2,000 20.4 / 23.0).
+_LOCKED_MIN, _LOCKED_MAX = 64 << 10, 64 << 20
 
 
 def _give_back(ptr: int, pid: int) -> None:
