@@ -19,7 +19,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import re
-import weakref
+import sys
 from typing import Optional, Sequence
 
 import numpy as np
@@ -177,11 +177,20 @@ def _words(words: np.ndarray) -> np.ndarray:
 _LOCKED_MIN, _LOCKED_MAX = 64 << 10, 64 << 20
 
 
-def _give_back(ptr: int, pid: int) -> None:
-    # a forked child only has a copy, and of the cache's lock as well, which another
-    # thread of the parent may have held
-    if os.getpid() == pid:
-        lib().flk_host_free(ptr)
+class _Block:
+    """A page-locked block under an array; goes back with the last reference."""
+
+    __slots__ = ("__array_interface__", "ptr", "pid")
+
+    def __init__(self, ptr: int, n: int):
+        self.ptr, self.pid = ptr, os.getpid()
+        self.__array_interface__ = {"data": (ptr, False), "shape": (n, WORDS), "typestr": "<f4", "version": 3}
+
+    def __del__(self, getpid=os.getpid, finalizing=sys.is_finalizing):
+        # a forked child only has a copy, and of the cache's lock as well, which
+        # another thread of the parent may have held
+        if getpid() == self.pid and not finalizing():
+            lib().flk_host_free(self.ptr)
 
 
 def _result(n: int) -> np.ndarray:
@@ -192,9 +201,7 @@ def _result(n: int) -> np.ndarray:
     if _LOCKED_MIN <= nbytes <= _LOCKED_MAX:
         p = C.c_void_p()
         if lib().flk_host_alloc(nbytes, C.byref(p)) == FLK_OK:
-            block = (C.c_char * nbytes).from_address(p.value)
-            weakref.finalize(block, _give_back, p.value, os.getpid()).atexit = False
-            return np.frombuffer(block, dtype=np.float32).reshape(n, WORDS)
+            return np.asarray(_Block(p.value, n))
     return np.empty((n, WORDS), dtype=np.float32)
 
 
