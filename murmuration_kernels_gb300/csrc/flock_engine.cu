@@ -302,7 +302,7 @@ bool host_free(void* p) {
     return true;
 }
 
-// An engine's control block: page-locked, or ordinary memory where the host locks
+// An engine's control blocks, out and in: page-locked, or ordinary memory where the host locks
 // no more (its copies then return when they are done).
 static uint8_t* control_alloc(size_t bytes) {
     void* p = host_alloc(bytes);
@@ -435,7 +435,6 @@ Engine::~Engine() {
     dfree(status_); dfree(sets_);
     dfree(block_); dfree(staging_); dfree(inv_);
     control_free(h_up_);
-    control_free(h_down_);
     host_free(h_bounce_);
     dfree(dec64_); dfree(out64_); dfree(active_); dfree(err64_);
     stream_put(device_, copy_);
@@ -670,7 +669,7 @@ std::vector<int> Engine::flock_ids() const {
 // page-locked host block each way, so that a call waits for the GPU once: the
 // steps, then one copy of the error word, clocks and countdowns.
 void Engine::ensure_block(uint32_t flocks) {
-    if (h_down_ && flocks <= table_cap_) return;
+    if (h_up_ && flocks <= table_cap_) return;
     const uint32_t cap = std::max(flocks, table_cap_ * 2);
     const size_t bytes = BLOCK_TABLE + (size_t)cap * sizeof(FlockDesc);
     size_t acct = 0;
@@ -685,9 +684,8 @@ void Engine::ensure_block(uint32_t flocks) {
     table_cap_ = cap;
     FLK_CUDA(cudaStreamSynchronize(stream_));  // the last upload has left its host block
     control_free(h_up_);
-    control_free(h_down_);
-    h_up_ = control_alloc(bytes);
-    h_down_ = control_alloc(bytes);
+    h_up_ = control_alloc(2 * bytes);
+    h_down_ = h_up_ + bytes;
     ctl_seen_ = false;
     free_graphs();
 }

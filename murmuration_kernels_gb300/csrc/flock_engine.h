@@ -277,8 +277,8 @@ private:
     std::vector<int> table_ids_;
     FlockDesc* table_d_ = nullptr;  // in block_
     uint32_t table_cap_ = 0;
-    // the control block and, BLOCK_TABLE bytes on, the flock table; the page-locked
-    // blocks its contents go out from and come back to
+    // the control block and, BLOCK_TABLE bytes on, the flock table; the host blocks
+    // (halves of one) its contents go out from and come back to
     static constexpr size_t BLOCK_TABLE = 256;
     uint8_t *block_ = nullptr, *h_up_ = nullptr, *h_down_ = nullptr;
     uint8_t* h_bounce_ = nullptr;   // bounce_block, and its device address
