@@ -355,7 +355,7 @@ def pass_bandwidths(r, n):
 # the step traffic in profiles/traffic_step_1m.txt are re-taken whenever the
 # kernels change.
 DECIDE_INST_1M = 50.1e6
-PROFILED_AT = "b10a817"
+PROFILED_AT = "23e2254"
 GB300_SMS = 152
 
 

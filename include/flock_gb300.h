@@ -56,8 +56,9 @@ typedef struct {
 int flk_open_host(int32_t device, uint32_t n, float time, const float* words, flk_flock** out);
 /* Reads a .flk file and uploads it (cuda/flock.cu:340-354). */
 int flk_open_file(int32_t device, const char* path, flk_flock** out);
-/* Advances `steps` steps (the step loop, cuda/flock.cu:453-470); returns
- * after the work is queued and checked (synchronises). */
+/* Advances `steps` steps (the step loop, cuda/flock.cu:453-470), launched as CUDA
+ * graphs of a step or of ten, or as one kernel for a small flock; returns after
+ * the work is done and checked (synchronises). */
 int flk_step(flk_flock* f, uint32_t steps);
 /* Same, launched pass by pass with CUDA events; fills the per-pass means of
  * the last steps-warmup steps (cuda/flock.cu:447-492). */
@@ -103,8 +104,9 @@ int flk_step_f64(flk_flock* f, double* out64, double* report);
  * at a time; before each step it overwrites a `flush_bytes` device buffer so
  * the step starts with a cold L2, then brackets the step with CUDA events on
  * the library's stream. ms_per_step[steps] receives each step's device time.
- * Each step runs as in flk_step's multi-step runs: its integrate also counts
- * the next step's grid. The first grid is counted before the first timed step
+ * Each step runs as in flk_step's multi-step runs of the separate kernels: its
+ * integrate also counts the next step's grid (a small flock, which flk_step runs
+ * in one kernel, gets the same bits here). The first grid is counted before the first timed step
  * and one untimed step follows the last, so the flock advances steps + 1. */
 int flk_time_steps(flk_flock* f, uint32_t steps, uint64_t flush_bytes, float* ms_per_step);
 /* flk_batch_tune_cell for a plain flock. */
@@ -128,7 +130,7 @@ int flk_batch_create(int32_t device, flk_batch** out);
 int flk_batch_add(flk_batch* b, uint32_t n, float time, const float* words, int32_t* id);
 /* Drops a flock and frees its storage for later flocks; no counterpart. */
 int flk_batch_remove(flk_batch* b, int32_t id);
-/* Advances every flock in the batch by `steps` steps (10-step CUDA graphs). */
+/* Advances every flock in the batch by `steps` steps (as flk_step). */
 int flk_batch_step(flk_batch* b, uint32_t steps);
 /* Steps only the listed flocks, each by its own count (0 = idle). */
 int flk_batch_step_each(flk_batch* b, const int32_t* ids, const uint32_t* steps, uint32_t count);
@@ -158,7 +160,7 @@ int flk_batch_tune(flk_batch* b, int32_t stream_bps, int32_t decide_bps, int32_t
  * the reference's cell is a compile-time constant. */
 int flk_batch_tune_cell(flk_batch* b, float cell_m);
 /* Which decide kernel steps without grid output run (0, the default, sweeps
- * the cell-ordered state through the caches; 1 stages each CTA's
+ * the cell-ordered positions through the caches; 1 stages each CTA's
  * neighbourhood in shared memory with TMA bulk copies first, falling back to
  * the direct sweep where birds of several flocks meet). Both find the same
  * neighbours and give the same decisions; sums may differ by rounding. Other

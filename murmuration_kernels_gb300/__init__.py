@@ -365,7 +365,7 @@ class Flock:
         _check(lib().flk_tune_cell(self._h, C.c_float(cell)))
 
     def tune_decide(self, staged: int) -> None:
-        """The production decide kernel: 0 sweeps the state, 1 stages cells in shared memory."""
+        """The production decide kernel: 0 sweeps the positions, 1 stages them in shared memory."""
         _check(lib().flk_tune_decide(self._h, staged))
 
     def debug_scan_timeout(self, skip_tile: int = 0, spin_limit: int = 1000) -> None:

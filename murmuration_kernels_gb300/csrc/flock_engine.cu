@@ -1190,8 +1190,10 @@ void Engine::enqueue_steps(uint32_t n) {
 
 // CTAs per flock where the table's flocks all run as one cluster each (k_small), or
 // 0: the largest cluster of which all the flocks' are on the chip together, if its
-// threads are as many as the largest flock's birds. Measured against the separate
-// kernels where each size takes over (us a step): 9 flocks of 1,000 birds (16 CTAs)
+// threads are as many as the largest flock's birds. How many clusters fit depends on
+// the GPU's own layout (one GB300 holds nine of 16 CTAs, 18 of 8, 36 of 4, 74 of 2;
+// another 7, 15, 36, 76), so it is asked for. Measured against the separate kernels
+// on the former where each size takes over (us a step): 9 flocks of 1,000 birds (16 CTAs)
 // 9.7 / 21.1, of 4,000 20.7 / 26.2; 18 flocks (8) of 1,000 11.6 / 22.6, of 4,000
 // 32 / 32; 20 flocks (4) of 2,000 18.8 / 28.3; 37 flocks (2) of 1,000 17.2 / 27.5;
 // 150 flocks (1) of 500 15.9 / 33.9. Clusters in a second turn take as long again.

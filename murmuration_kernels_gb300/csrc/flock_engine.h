@@ -97,7 +97,7 @@ struct LaunchShape {
     int graph_chunk = 10;           // steps per captured CUDA graph
     size_t decide_extra_smem = 0;   // dynamic shared memory reserved beyond decide's own (occupancy experiments)
     float cell = 4.0f;              // production cell edge (m); any edge gives the same neighbour sets
-    int decide_kind = 0;            // production decide: 0 sweeps the state, 1 stages cells in shared memory
+    int decide_kind = 0;            // production decide: 0 sweeps the view, 1 stages its rows in shared memory
 };
 
 struct GridDebug {  // host copies of one step's grid and neighbour-set summaries

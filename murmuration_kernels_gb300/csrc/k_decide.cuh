@@ -112,7 +112,9 @@ __device__ __forceinline__ RowBox row_box(const Bird& b, float r, uint32_t bucke
               nz = pcell(b.p.z + q.reach, inv_row) - q.lz + 1;
     q.bits = row_bits(buckets);
     const uint32_t bx = q.bits & 31u, by = (q.bits >> 5) & 31u, bz = q.bits >> 10;
-    // the first test keeps the cell numbers far from overflow (and fails for NaN)
+    // the first test keeps the cell numbers far from overflow (an infinite or NaN
+    // radius fails it; a NaN coordinate alone does not, and needs not: every
+    // distance to such a bird is NaN and fails its own test)
     const float far = fmaxf(fabsf(b.p.x), fmaxf(fabsf(b.p.y), fabsf(b.p.z))) + q.reach;
     q.lattice = far * inv_x < 1e9f && nx <= (1 << bx) && ny <= (1 << by) && nz <= (1 << bz);
     q.ny = (uint32_t)ny;

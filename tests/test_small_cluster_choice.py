@@ -1,6 +1,6 @@
 """Which batches run as one cluster per flock, of how many thread blocks, and that
 each cluster size runs and gives the separate kernels' bits. How many clusters of
-each size fit on the GPU at once is the device's own (eight or nine of 16 blocks on
+each size fit on the GPU at once is the device's own (seven to nine of 16 blocks on
 the GB300s seen), so the counts on both sides of each line are taken from it. And
 the autotuner's knobs where the launch shapes have no effect."""
 from __future__ import annotations
