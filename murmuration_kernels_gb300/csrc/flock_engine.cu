@@ -1296,11 +1296,14 @@ void Engine::launch_graph(const StepGraph& sg) {
 // cheap to capture (five nodes), so any run of a few steps goes through it. A
 // graph of a whole chunk has no gap between its steps (us a step, step graphs
 // against chunk graphs: 8,193 birds 26.0 / 23.7, 37,501 29.6 / 26.3, 100,000
-// 31.7 / 27.7, 300,000 45.6 / 42.7, 1M 109 / 105); it is built for runs of ten
-// chunks and for the third run of a table that stays the same, a served pool's
-// chunks among them (its median latency under a Poisson load 14.8 -> 13.5 ms),
-// while the GPU is busy with a chunk. The launches are the captured ones, so the
-// results are the same.
+// 31.7 / 27.7, 300,000 45.6 / 42.7, 1M 109 / 105), but each of its launches moves
+// the state, not one step in MOVE_EVERY (chunks of one step: 1M 134 / 136, 3M 324 /
+// 346; of two: 3M 308 / 310, 16.7M 1,526 / 1,596; of ten: 3M 291 / 289, 16.7M 1,490 /
+// 1,491). It is built for runs of ten chunks and, up to a million birds per step of
+// a chunk, for the third run of a table that stays the same, a served pool's chunks
+// among them (its median latency under a Poisson load 14.8 -> 13.5 ms), while the
+// GPU is busy with a chunk. The launches are the captured ones, so the results are
+// the same.
 void Engine::enqueue_run(uint32_t steps) {
     if (const uint32_t ctas = small_ctas()) {
         enqueue_small(steps, ctas);
@@ -1311,7 +1314,7 @@ void Engine::enqueue_run(uint32_t steps) {
     uint32_t done = 0;
     if (steps >= chunk) {
         const bool ready = chunk_graph_.exec && chunk_graph_.steps == chunk && !chunk_graph_.stale;
-        if (ready || steps >= 10 * chunk || same_runs_ >= 2) {
+        if (ready || steps >= 10 * chunk || (same_runs_ >= 2 && V_ / 1000000u <= chunk)) {
             if (!ready) {
                 enqueue_singly(chunk);
                 done = chunk;
