@@ -546,7 +546,7 @@ struct Snapshot {
     float* words;
     float time = 0.f;
     uint32_t steps_done = 0;
-    int state = 0;  // 0 pending, 1 landed, <0 error
+    int state = 0;  // 0 pending, 1 landed, 2 the request left before it was taken, <0 error
 };
 }  // namespace
 
@@ -644,7 +644,7 @@ void flk_pool::loop() {
                     const auto it = std::find(live.begin(), live.end(), sn->r);
                     Retire x{sn->r, nullptr, 0.f, err != 0, sn};
                     FLK_CUDA_ABI(cudaEventCreateWithFlags(&x.done, cudaEventDisableTiming));
-                    if (it == live.end() || err) {  // never for a resident request; fail rather than wait
+                    if (it == live.end() || err) {  // (the former never: see the end of the boundary)
                         x.failed = true;
                         FLK_CUDA_ABI(cudaEventRecord(x.done, eng->stream()));
                     } else {
@@ -674,6 +674,17 @@ void flk_pool::loop() {
                     retiring.push_back(x);
                 }
                 stats.resident_bytes = resident_bytes;
+                // snapshots asked for during this boundary of requests that it retired:
+                // no later boundary has them, and there may be none
+                for (size_t k = 0; k < snaps.size();) {
+                    if (std::find(resident.begin(), resident.end(), snaps[k]->r) != resident.end()) {
+                        ++k;
+                        continue;
+                    }
+                    snaps[k]->state = 2;
+                    snaps.erase(snaps.begin() + k);
+                    cv_done.notify_all();
+                }
                 if (!done.empty()) cv_retire.notify_all();
             }
             bool any;
@@ -820,30 +831,35 @@ extern "C" int flk_pool_snapshot(flk_pool* p, uint64_t ticket, float* words, flo
     if (it == p->reqs.end()) return fail(FLK_ERR_ID, "flk_pool_snapshot: unknown ticket");
     auto r = it->second;
     if (r->n && !words) return fail(FLK_ERR_ARG, "flk_pool_snapshot: null words");
-    if (r->state == 1 && std::find(p->resident.begin(), p->resident.end(), r) == p->resident.end())
-        p->cv_done.wait(lk, [&] { return r->state != 1 || p->stop; });  // retiring: its result is landing
-    if (r->state < 0) return fail(r->state, "flk_pool_snapshot: request failed: " + p->worker_error);
-    if (r->state == 1 && p->stop) return fail(FLK_ERR_CUDA, "flk_pool_snapshot: pool stopped");
     float t = 0.f;
     uint32_t k = 0;
     const size_t bytes = (size_t)r->n * flk::WORDS * 4;
-    if (r->state == 0) {  // still queued: its input state
-        if (bytes) std::memcpy(words, r->words, bytes);
-        t = r->time;
-    } else if (r->state == 2) {  // finished: its result
-        if (bytes) std::memcpy(words, r->out_words, bytes);
-        t = r->result_time;
-        k = r->steps;
-    } else {  // resident: taken at the next chunk boundary while the others keep running
-        auto sn = std::make_shared<Snapshot>();
-        sn->r = r;
-        sn->words = words;
-        p->snaps.push_back(sn);
-        p->cv_work.notify_one();
-        p->cv_done.wait(lk, [&] { return sn->state != 0 || p->stop; });
-        if (sn->state != 1) return fail(sn->state ? sn->state : FLK_ERR_CUDA, "flk_pool_snapshot: copy failed");
-        t = sn->time;
-        k = sn->steps_done;
+    for (bool taken = false; !taken;) {  // again where the request left before its boundary
+        if (r->state == 1 && std::find(p->resident.begin(), p->resident.end(), r) == p->resident.end())
+            p->cv_done.wait(lk, [&] { return r->state != 1 || p->stop; });  // retiring: its result is landing
+        if (r->state < 0) return fail(r->state, "flk_pool_snapshot: request failed: " + p->worker_error);
+        if (r->state == 1 && p->stop) return fail(FLK_ERR_CUDA, "flk_pool_snapshot: pool stopped");
+        taken = true;
+        if (r->state == 0) {  // still queued: its input state
+            if (bytes) std::memcpy(words, r->words, bytes);
+            t = r->time;
+        } else if (r->state == 2) {  // finished: its result
+            if (bytes) std::memcpy(words, r->out_words, bytes);
+            t = r->result_time;
+            k = r->steps;
+        } else {  // resident: taken at the next chunk boundary while the others keep running
+            auto sn = std::make_shared<Snapshot>();
+            sn->r = r;
+            sn->words = words;
+            p->snaps.push_back(sn);
+            p->cv_work.notify_one();
+            p->cv_done.wait(lk, [&] { return sn->state != 0 || p->stop; });
+            taken = sn->state != 2;
+            if (taken && sn->state != 1)
+                return fail(sn->state ? sn->state : FLK_ERR_CUDA, "flk_pool_snapshot: copy failed");
+            t = sn->time;
+            k = sn->steps_done;
+        }
     }
     lk.unlock();
     if (time) *time = t;
